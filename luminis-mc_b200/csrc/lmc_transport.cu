@@ -961,32 +961,46 @@ static lmc_status sweep_adjoint_layout(const lmc_handle *h, const lmc_adjoint_op
 // Absorption recorder (the variants with their code; the others leave it out).
 using KernelFn = void (*)(const lmc::dev::Scene *, lmc::dev::RunParams);
 
+// E: extras; T = false: the variants without the reverse-path history (queued runs only).
+template <bool E, bool T>
+static KernelFn pick_transport_t(bool fp32, bool wide, bool adj, bool sw)
+{
+  using namespace lmc::dev;
+  if (sw && adj)
+    return fp32 ? transport_kernel<float, true, 3, true, true, false, false, T>
+                : transport_kernel<double, true, 1, true, true, false, false, T>;
+  if (sw)
+    return fp32 ? transport_kernel<float, true, 3, false, true, false, E, T>
+                : transport_kernel<double, true, 2, false, true, false, E, T>;
+  if (adj)
+    return fp32 ? transport_kernel<float, true, 3, true, false, false, false, T>
+                : transport_kernel<double, true, 1, true, false, false, false, T>;
+  if (fp32)
+    return wide ? transport_kernel<float, true, 4, false, false, false, E, T>
+                : transport_kernel<float, true, 2, false, false, false, E, T>;
+  return transport_kernel<double, true, 2, false, false, false, E, T>;
+}
+
 template <bool E>
-static KernelFn pick_transport_e(bool fp32, bool queued, bool wide, bool adj, bool sw, bool est)
+static KernelFn pick_transport_e(bool fp32, bool queued, bool wide, bool adj, bool sw, bool est, bool track)
 {
   using namespace lmc::dev;
   if (est)
     return fp32 ? transport_kernel<float, true, 2, false, false, true, E>
                 : transport_kernel<double, true, 2, false, false, true, E>;
-  if (sw && adj)
-    return fp32 ? transport_kernel<float, true, 3, true, true> : transport_kernel<double, true, 1, true, true>;
-  if (sw)
-    return fp32 ? transport_kernel<float, true, 3, false, true, false, E>
-                : transport_kernel<double, true, 2, false, true, false, E>;
-  if (adj)
-    return fp32 ? transport_kernel<float, true, 3, true> : transport_kernel<double, true, 1, true>;
-  if (fp32)
-    return queued ? (wide ? transport_kernel<float, true, 4, false, false, false, E>
-                           : transport_kernel<float, true, 2, false, false, false, E>)
-                  : transport_kernel<float, false, 1, false, false, false, E>;
-  return queued ? transport_kernel<double, true, 2, false, false, false, E>
+  if (!queued)
+    return fp32 ? transport_kernel<float, false, 1, false, false, false, E>
                 : transport_kernel<double, false, 1, false, false, false, E>;
+  return track ? pick_transport_t<E, true>(fp32, wide, adj, sw)
+               : pick_transport_t<E, false>(fp32, wide, adj, sw);
 }
 
-static KernelFn pick_transport(bool fp32, bool queued, bool wide, bool adj, bool sw, bool est, bool extras)
+// track: the launch keeps the reverse-path history, stages tables or writes records.
+static KernelFn pick_transport(bool fp32, bool queued, bool wide, bool adj, bool sw, bool est, bool extras,
+                               bool track)
 {
-  return extras ? pick_transport_e<true>(fp32, queued, wide, adj, sw, est)
-                : pick_transport_e<false>(fp32, queued, wide, adj, sw, est);
+  return extras ? pick_transport_e<true>(fp32, queued, wide, adj, sw, est, track)
+                : pick_transport_e<false>(fp32, queued, wide, adj, sw, est, track);
 }
 
 template <int kT>
@@ -1251,7 +1265,6 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     extras = extras || scene_extras(sw ? h->scenes[k] : h->scene);
   if (adj && extras)                     // (MixtureLayers are refused by the layout already)
     return fail(LMC_ERR_UNSUPPORTED, "likelihood-ratio runs do not record an Absorption grid");
-  const KernelFn tk = pick_transport(fp32, h->queued, wide, adj != nullptr, sw, est, extras);
   TallyLaunch tl{};
   if (h->queued && h->tally_doubles > 0) {
     const lmc_status st = tally_setup(opts->tally_mode, sw, fp32, adj != nullptr,
@@ -1269,7 +1282,15 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   const bool replay = h->queued && !est && !opts->records && !opts->no_replay &&
                       opts->track_reverse_paths && any_cbs;
   rp.cbs_replay = replay ? 1 : 0;
-  if (replay) {                          // no history: the ring and first species only
+  const bool track = !h->queued || est || opts->records || opts->stage_tables || (any_cbs && !replay);
+  // StatisticsSensors read the penetration depth, which the variants without history carry
+  // beside the extras only
+  bool any_stat = false;
+  for (int k = 0; k < h->n_scenes; ++k)
+    any_stat = any_stat || (sw ? h->scenes[k] : h->scene).stat_mask != 0;
+  const KernelFn tk = pick_transport(fp32, h->queued, wide, adj != nullptr, sw, est,
+                                     extras || (!track && !adj && any_stat), track || (adj && any_stat));
+  if (replay || !track) {                // no history: the ring and first species only
     rp.track_reverse = 0;
     dyn_transport = fp32 ? dev::side_slim_bytes<float>() : dev::side_slim_bytes<double>();
   }
@@ -2143,7 +2164,7 @@ extern "C" lmc_status lmc_run_noalloc(const lmc_scene *s, uint64_t seed, uint64_
     return fail(LMC_ERR_INVALID, "block_size must be a multiple of 32 and at most 256");
   // the kernels lmc_run picks for the same scene and options
   const bool wide = fp32 && queued && (opts->blocks_per_sm == 0 || opts->blocks_per_sm >= 3);
-  const KernelFn tk = pick_transport(fp32, queued, wide, false, false, false, scene_extras(sc));
+  const KernelFn tk = pick_transport(fp32, queued, wide, false, false, false, scene_extras(sc), true);
   TallyLaunch tl{};
   if (queued && s->n_sensors > 0) {
     const lmc_status st = tally_setup(opts->tally_mode, false, fp32, false, sc, sensor_count, device,

@@ -1,0 +1,67 @@
+"""The transport's compiled variants against one another.
+
+A queued run without reverse-path history, staged tables or records takes variants with
+that code left out; `stage_tables` and `no_replay` select the general ones.  Both must give
+the same tallies and counts: binary64 to 1e-12 of each sensor's largest bin (order of the
+sums), binary32 to 1e-5 of it (separate compilations may round a binary32 operation
+differently; every photon keeps its discrete history, so counts are equal).
+"""
+import numpy as np
+import pytest
+
+import luminis_mc_b200 as lm
+from luminis_mc_b200 import workloads as W
+from luminis_mc_b200.device import DeviceRun
+
+pytestmark = pytest.mark.gpu
+TOL = {"fp64": 1e-12, "fp32": 1e-5}
+
+
+def _fluence_only(n):                 # no CBS sensor: nothing to replay
+    spec = W.bilayer_rgd_mie(n, 3)
+    spec["sensors"] = spec["sensors"][1:]
+    return spec
+
+
+def _statistics(n):                   # the penetration depth rides along
+    spec = W.mie_cbs_small(n, 4)
+    spec["sensors"].append({"kind": "statistics", "z": 0.0, "absorb": True, "events": 200,
+                            "theta": [0.0, 1.6, 16], "depth": [2.0, 64]})
+    return spec
+
+
+def _mixture_absorption(n):
+    spec = W.mixture_bilayer(n, 5)
+    spec["absorption"] = {"radius": 5.0, "depth": 2.0, "d_r": 0.25, "d_z": 0.1}
+    return spec
+
+
+def run_tallies(spec, precision, **options):
+    cfg, _, keep = W.build(lm, spec)
+    run = DeviceRun(cfg)
+    stats, _ = run.run(spec["n_photons"], spec["seed"], precision=precision, **options)
+    out = [t.copy() for t in run.host_tallies()]
+    grid = run.host_absorption()
+    run.close()
+    return stats, out + ([] if grid is None else [grid.copy()])
+
+
+def assert_same_run(a, b, tol):
+    (sa, ta), (sb, tb) = a, b
+    for key in ("photons", "events", "steps", "draws", "hits", "detected", "escaped", "stack",
+                "roulette", "cap", "error_flags"):
+        assert sa[key] == sb[key], key
+    assert len(ta) == len(tb)
+    for x, y in zip(ta, tb):
+        np.testing.assert_allclose(x, y, rtol=0, atol=tol * max(np.abs(y).max(), 1e-300))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("make", [_fluence_only, _statistics, _mixture_absorption],
+                         ids=["fluence_only", "statistics", "mixture_absorption"])
+def test_variants_without_history_equal_the_general_ones(make, precision, cuda):
+    spec = make(12_001)
+    default = run_tallies(spec, precision)
+    assert default[0]["events"] > 0
+    for options in ({"stage_tables": True}, {"no_replay": True, "stage_tables": True}):
+        assert_same_run(run_tallies(spec, precision, **options), default, TOL[precision])
