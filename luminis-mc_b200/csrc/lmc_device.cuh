@@ -199,9 +199,13 @@ struct AdjScene {
   unsigned long long cbs_off[LMC_MAX_SENSORS];
 };
 
+// Philox key increments per round.
+constexpr uint32_t kPhiloxStep0 = 0x9E3779B9u, kPhiloxStep1 = 0xBB67AE85u;
+
 struct RunParams {
   unsigned long long photon_begin, n_photons;
-  uint32_t key0, key1;
+  uint32_t key0, key1;                   // Philox key: the seed
+  uint32_t round_key[20];                // its ten rounds' keys (set_seed)
   int max_events, track_reverse;
   double *tallies;
   lmc_record *records;                   // this launch's photons: photon_begin + i at records[i]

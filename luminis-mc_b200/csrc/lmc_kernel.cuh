@@ -145,24 +145,30 @@ template <int kStride> struct RngT {
 using Rng = RngT<kBlock>;
 
 // The ten rounds of one block, inlined where the ring is filled: at the once-per-event
-// prefetch and at a draw that finds the ring dry.
+// prefetch and at a draw that finds the ring dry.  kKeys: the round keys are read from the
+// launch parameters (constant-bank operands) instead of being stepped with two adds a
+// round: 2 M binary64 bilayer photons 48.8 -> 46.0 ms, 2 M mixture photons 33.1 -> 31.9 ms,
+// 3 M with derivatives 49.7 -> 48.1 ms.  The plain binary32 transport (170 against 178 ms
+// for 20 M bilayer photons) and the sweeps (103.7 against 106 ms) step them: there the
+// 64- and 80-register allocations come out worse with the table.
+template <bool kKeys>
 __device__ __forceinline__ uint4 philox_block(uint32_t block, uint32_t p_lo, uint32_t p_hi,
-                                              uint32_t key0, uint32_t key1)
+                                              const RunParams &rp)
 {
   uint32_t c0 = block, c1 = 0u, c2 = p_lo, c3 = p_hi;
-  uint32_t k0 = key0, k1 = key1;
+  uint32_t k0 = rp.key0, k1 = rp.key1;
 #pragma unroll
   for (int r = 0; r < 10; ++r) {
     const uint32_t lo0 = 0xD2511F53u * c0, hi0 = __umulhi(0xD2511F53u, c0);
     const uint32_t lo1 = 0xCD9E8D57u * c2, hi1 = __umulhi(0xCD9E8D57u, c2);
-    const uint32_t n0 = hi1 ^ c1 ^ k0;
-    const uint32_t n2 = hi0 ^ c3 ^ k1;
+    const uint32_t n0 = hi1 ^ c1 ^ (kKeys ? rp.round_key[2 * r] : k0);
+    const uint32_t n2 = hi0 ^ c3 ^ (kKeys ? rp.round_key[2 * r + 1] : k1);
     c0 = n0;
     c1 = lo1;
     c2 = n2;
     c3 = lo0;
-    k0 += 0x9E3779B9u;
-    k1 += 0xBB67AE85u;
+    k0 += kPhiloxStep0;
+    k1 += kPhiloxStep1;
   }
   return make_uint4(c0, c1, c2, c3);
 }
@@ -186,9 +192,9 @@ template <int S> __device__ __forceinline__ void rng_reset(RngT<S> &g, unsigned 
 }
 
 // Generate the next block into the ring (words filled .. filled + 3).
-template <int S> __device__ __forceinline__ void rng_fill(RngT<S> &g, const RunParams &rp)
+template <bool kKeys, int S> __device__ __forceinline__ void rng_fill(RngT<S> &g, const RunParams &rp)
 {
-  const uint4 b = philox_block(g.filled >> 2, g.p_lo, g.p_hi, rp.key0, rp.key1);
+  const uint4 b = philox_block<kKeys>(g.filled >> 2, g.p_lo, g.p_hi, rp);
   g.word(g.filled) = b.x;
   g.word(g.filled + 1u) = b.y;
   g.word(g.filled + 2u) = b.z;
@@ -198,23 +204,24 @@ template <int S> __device__ __forceinline__ void rng_fill(RngT<S> &g, const RunP
 
 // Top the ring up (call while converged): up to two blocks, as long as a whole
 // block fits behind the words not yet consumed.
-template <typename R, int S> __device__ __forceinline__ void rng_prefetch(RngT<S> &g, const RunParams &rp)
+template <typename R, bool kKeys, int S>
+__device__ __forceinline__ void rng_prefetch(RngT<S> &g, const RunParams &rp)
 {
   const uint32_t used = g.draw * words_per_draw<R>(rp);
 #pragma unroll 1
   for (int i = 0; i < 2; ++i)
     if (g.filled + 4u <= used + kRing)
-      rng_fill(g, rp);
+      rng_fill<kKeys>(g, rp);
 }
 
 // Words of the next draw; generates a block only if the ring ran dry.
-template <typename R, int S> __device__ __forceinline__ void rng_words(RngT<S> &g, const RunParams &rp,
-                                                                       uint32_t &lo, uint32_t &hi)
+template <typename R, bool kKeys, int S>
+__device__ __forceinline__ void rng_words(RngT<S> &g, const RunParams &rp, uint32_t &lo, uint32_t &hi)
 {
   const uint32_t wpd = words_per_draw<R>(rp);
   const uint32_t w0 = g.draw * wpd;
   if (w0 + wpd > g.filled)
-    rng_fill(g, rp);
+    rng_fill<kKeys>(g, rp);
   lo = g.word(w0);
   hi = wpd == 2u ? g.word(w0 + 1u) : 0u;
   g.draw++;
@@ -236,10 +243,11 @@ template <> __device__ __forceinline__ double words_uniform<double>(const RunPar
   return __ull2double_rn(2ull * (w >> 12) + 1ull) * 1.1102230246251565e-16;   // 2^-53
 }
 
-template <typename R, int S> __device__ __forceinline__ R uniform(RngT<S> &g, const RunParams &rp)
+template <typename R, bool kKeys = false, int S>
+__device__ __forceinline__ R uniform(RngT<S> &g, const RunParams &rp)
 {
   uint32_t lo, hi;
-  rng_words<R>(g, rp, lo, hi);
+  rng_words<R, kKeys>(g, rp, lo, hi);
   return words_uniform<R>(rp, lo, hi);
 }
 
@@ -301,9 +309,28 @@ template <typename R> __host__ __device__ constexpr size_t side_slim_bytes()
   return (sizeof(uint32_t) * kRing * kBlock + sizeof(int) * kBlock + 15) & ~size_t(15);
 }
 
-struct Counters {
-  uint32_t events, steps, draws;
+// A thread's counts of a run.  kOn = false: not kept per event (see transport_kernel).
+template <bool kOn> struct Counters {
+  uint32_t events = 0, steps = 0, draws = 0;
+  __device__ __forceinline__ void step() { steps++; }
+  __device__ __forceinline__ void event() { events++; }
 };
+template <> struct Counters<false> {
+  __device__ __forceinline__ void step() {}
+  __device__ __forceinline__ void event() {}
+};
+
+// A 64-bit sum in two 32-bit words of shared memory: native adds, where a 64-bit shared
+// add is a retry loop.
+__device__ __forceinline__ void add_wide(unsigned *sum, unsigned v)
+{
+  if (atomicAdd(&sum[0], v) + v < v)
+    atomicAdd(&sum[1], 1u);
+}
+__device__ __forceinline__ unsigned long long wide(const unsigned *sum)
+{
+  return ((unsigned long long)sum[1] << 32) | sum[0];
+}
 
 // ------------------------------------------------------- likelihood-ratio score
 // Score of a photon history: d/d(param) of log(path density x weight), summed over
@@ -2151,17 +2178,18 @@ __device__ __forceinline__ void record_absorption_f32(const AbsorbGrid &g, doubl
 // replay) leaves the sensor planes out: a replayed event never reaches one, because
 // crossing a plane at z <= 0 ends a photon.  kTrack = false (see transport_kernel) leaves
 // the reverse-path history and, without kExtras, the penetration depth out.
-template <typename R, bool kQueue, bool kAdj, bool kExtras = false, bool kHits = true, bool kTrack = true>
+template <typename R, bool kQueue, bool kAdj, bool kExtras = false, bool kHits = true, bool kTrack = true,
+          bool kKeys = false, bool kCount = true>
 __device__ __forceinline__ int event_move(const Scene &sc, const RunParams &rp, Photon<R> &ph,
-                                          Side<R> &side, Flight<R> &fl, Counters &cnt,
+                                          Side<R> &side, Flight<R> &fl, Counters<kCount> &cnt,
                                           unsigned long long *s_hits, int &med_out)
 {
-  rng_prefetch<R>(ph.rng, rp);
+  rng_prefetch<R, kKeys>(ph.rng, rp);
   {
     // free path with the layer's mean free path (src/medium.cpp:123-126,
     // src/sample.cpp:90-94)
-    R step = -lay_mfp<R>(sc.layers[ph.layer]) * m_log(uniform<R>(ph.rng, rp));
-    cnt.steps++;
+    R step = -lay_mfp<R>(sc.layers[ph.layer]) * m_log(uniform<R, kKeys>(ph.rng, rp));
+    cnt.step();
     if (kAdj)
       flight_start<R>(sc, fl, sc.layers[ph.layer].medium);
     const R dx = ph.P[6], dy = ph.P[7], dz = ph.P[8];
@@ -2228,7 +2256,7 @@ __device__ __forceinline__ int event_move(const Scene &sc, const RunParams &rp, 
   const int lflags = SL.flags;
   int med_idx = SL.medium;
   if (kExtras && (lflags & kLayerMixture)) {
-    const double u = (double)uniform<R>(ph.rng, rp);
+    const double u = (double)uniform<R, kKeys>(ph.rng, rp);
     int i = 0;
     while (i < SL.n_species - 1 && sc.mix_cdf[SL.mix_begin + i] < u)
       ++i;
@@ -2245,14 +2273,14 @@ __device__ __forceinline__ int event_move(const Scene &sc, const RunParams &rp, 
 // absorption weight, roulette and the event cap.  kDeposit = false (the CBS replay)
 // leaves the Absorption recorder out: the transport recorded those deposits already.
 template <typename R, bool kAdj, bool kExtras = false, bool kDeposit = true, bool kTrack = true,
-          bool kStaged = true>
+          bool kStaged = true, bool kKeys = false, bool kCount = true>
 __device__ __forceinline__ int event_scatter(const Scene &sc, const RunParams &rp, Photon<R> &ph,
-                                             Side<R> &side, Flight<R> &fl, Counters &cnt, int med_idx)
+                                             Side<R> &side, Flight<R> &fl, Counters<kCount> &cnt, int med_idx)
 {
   const Layer &SL = sc.layers[ph.layer];
   const int lflags = SL.flags;
   const Medium &m = sc.media[med_idx];
-  const R theta = sample_theta<R>(m, uniform<R>(ph.rng, rp));  // :429
+  const R theta = sample_theta<R>(m, uniform<R, kKeys>(ph.rng, rp));  // :429
   Cx<R> S2, S1;
   amplitudes<R, kStaged>(m, theta, S2, S1);                            // :430
   // sample_phi_conditional (src/phase.cpp:27-49)
@@ -2324,12 +2352,12 @@ __device__ __forceinline__ int event_scatter(const Scene &sc, const RunParams &r
     for (;; ++trial) {
       if (trial == kMaxRejectionTrials)
         return kError;
-      const R u1 = uniform<R>(ph.rng, rp);
+      const R u1 = uniform<R, kKeys>(ph.rng, rp);
       m_sincos_turn(u1, &sp, &cp);
       const R F = a * cp * cp + b * sp * sp + c * cp * sp;
       const R Fc = F > R(0) ? F : R(0);
       Facc = F;
-      if (uniform<R>(ph.rng, rp) * Fmax <= Fc)
+      if (uniform<R, kKeys>(ph.rng, rp) * Fmax <= Fc)
         break;
     }
   }
@@ -2405,7 +2433,7 @@ __device__ __forceinline__ int event_scatter(const Scene &sc, const RunParams &r
     }
   }
   ph.events++;                                                // :578-587
-  cnt.events++;
+  cnt.event();
   if (kExtras && kDeposit && (lflags & kLayerAbsorb)) {       // :589-592
     const double t = sc.absorb.d_t > 0.0 ? launch_time<R>(sc, rp, ph) + ph.opath : 0.0;  // velocity 1
     const double dw = SL.mu_t > 0 ? ph.w * SL.absorb_prob : 1.0;
@@ -2416,7 +2444,7 @@ __device__ __forceinline__ int event_scatter(const Scene &sc, const RunParams &r
   }
   ph.w *= SL.albedo;                                          // the layer's aggregate albedo
   if (ph.w < 1e-4) {                                          // :596-607
-    if (uniform<R>(ph.rng, rp) < R(0.1))
+    if (uniform<R, kKeys>(ph.rng, rp) < R(0.1))
       ph.w /= 0.1;
     else
       return kRoulette;
@@ -2428,17 +2456,18 @@ __device__ __forceinline__ int event_scatter(const Scene &sc, const RunParams &r
 
 // One loop iteration of run_photon (src/simulation.cpp:297-614).  Returns the photon's
 // fate (kAlive if it continues).
-template <typename R, bool kQueue, bool kAdj, bool kExtras = false, bool kTrack = true, bool kStaged = true>
+template <typename R, bool kQueue, bool kAdj, bool kExtras = false, bool kTrack = true, bool kStaged = true,
+          bool kKeys = false, bool kCount = true>
 __device__ __forceinline__ int event_step(const Scene &sc, const RunParams &rp, Photon<R> &ph,
-                                          Side<R> &side, Flight<R> &fl, Counters &cnt,
+                                          Side<R> &side, Flight<R> &fl, Counters<kCount> &cnt,
                                           unsigned long long *s_hits)
 {
   int med_idx = 0;
   const int fate =
-      event_move<R, kQueue, kAdj, kExtras, true, kTrack>(sc, rp, ph, side, fl, cnt, s_hits, med_idx);
+      event_move<R, kQueue, kAdj, kExtras, true, kTrack, kKeys>(sc, rp, ph, side, fl, cnt, s_hits, med_idx);
   if (fate != kAlive)
     return fate;
-  return event_scatter<R, kAdj, kExtras, true, kTrack, kStaged>(sc, rp, ph, side, fl, cnt, med_idx);
+  return event_scatter<R, kAdj, kExtras, true, kTrack, kStaged, kKeys>(sc, rp, ph, side, fl, cnt, med_idx);
 }
 
 template <typename R>
@@ -2544,14 +2573,24 @@ __device__ __forceinline__ int sweep_scene(const RunParams &rp, unsigned long lo
 // are replayed), stages no tables and writes no records, with the code for all three left
 // out rather than branched around at every event.  What bounds the event loop is issue and
 // instruction fetch, so the shorter loop shows: 20 M bilayer photons (binary32) 193.7 ->
-// 179.6 ms, 2 M mixture photons 36.0 -> 33.9 ms.
+// 179.6 ms, 2 M mixture photons 36.0 -> 33.1 ms.
+// kCount: each thread counts its events, flights and draws.  The 64-register kernels
+// (kMinBlocks 4) instead add a photon's events and draws to the block's sums when it ends
+// (every flight ends in an event or in one of the fates below): three registers fewer over
+// the loop, spills 48 -> 10 bytes, 20 M bilayer photons 179.5 -> 170.4 ms.  Kernels with
+// registers to spare lose 1-3 % to the adds and count per thread.
 template <typename R, bool kQueue, int kMinBlocks, bool kAdj = false, bool kSweep = false, bool kEst = false,
           bool kExtras = false, bool kTrack = true>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Scene *__restrict__ g_scene, RunParams rp)
 {
   __shared__ __align__(16) unsigned char s_raw[kSweep ? 16 : sizeof(Scene)];
   __shared__ unsigned long long s_hits[LMC_MAX_SENSORS];
-  __shared__ unsigned long long s_fate[7];
+  // a queued launch's photons fit its queue (fewer than 2^32); an inline launch has no bound
+  using Fates = std::conditional_t<kQueue, unsigned, unsigned long long>;
+  __shared__ Fates s_fate[7];
+  __shared__ unsigned s_events[2], s_draws[2];
+  constexpr bool kCount = kMinBlocks < 4;
+  constexpr bool kKeys = sizeof(R) == 8 || kAdj || kExtras;
   extern __shared__ __align__(16) unsigned char s_dyn[];
   Side<R> &side = *reinterpret_cast<Side<R> *>(s_dyn);
   Flight<R> fl;
@@ -2562,6 +2601,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
     s_hits[threadIdx.x] = 0;
   if (threadIdx.x < 7)
     s_fate[threadIdx.x] = 0;
+  if (threadIdx.x < 2)
+    s_events[threadIdx.x] = s_draws[threadIdx.x] = 0;
   double *s_est = reinterpret_cast<double *>(s_dyn + rp.side_off);
   if (kEst)
     for (int j = threadIdx.x; j < rp.est_smem_doubles; j += blockDim.x)
@@ -2574,7 +2615,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
   }
   const Scene *scp = kSweep ? g_scene : reinterpret_cast<const Scene *>(s_raw);
   const unsigned lane = threadIdx.x & 31u;
-  Counters cnt = {0, 0, 0};
+  Counters<kCount> cnt;
   Photon<R> ph;
   ph.rng.ring = &side.ring[0][threadIdx.x];
   bool alive = false, done = false;
@@ -2613,18 +2654,23 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
       // then the scatter
       int med_idx = 0;
       if (alive)
-        fate = event_move<R, kQueue, kAdj, kExtras>(*scp, rp, ph, side, fl, cnt, s_hits, med_idx);
+        fate = event_move<R, kQueue, kAdj, kExtras, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, s_hits, med_idx);
       estimate_warp<R>(*scp, rp, ph, side, med_idx, alive && fate == kAlive, s_hits, s_est);
       if (alive && fate == kAlive)
-        fate = event_scatter<R, kAdj, kExtras>(*scp, rp, ph, side, fl, cnt, med_idx);
+        fate = event_scatter<R, kAdj, kExtras, true, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, med_idx);
     } else if (alive) {
-      fate = event_step<R, kQueue, kAdj, kExtras, kTrack, kTrack && !kSweep>(*scp, rp, ph, side, fl, cnt, s_hits);
+      fate = event_step<R, kQueue, kAdj, kExtras, kTrack, kTrack && !kSweep, kKeys>(*scp, rp, ph, side, fl, cnt, s_hits);
     }
     if (alive) {
       if (fate != kAlive) {
         alive = false;
-        cnt.draws += ph.rng.draw;
-        atomicAdd(&s_fate[fate], 1ull);
+        if constexpr (kCount) {
+          cnt.draws += ph.rng.draw;
+        } else {
+          add_wide(s_events, ph.events);
+          add_wide(s_draws, ph.rng.draw);
+        }
+        atomicAdd(&s_fate[fate], Fates(1));
         if (kTrack && rp.records)
           write_record<R>(*scp, rp, ph, side, fate);
         if (fate == kError)
@@ -2634,31 +2680,39 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
       }
     }
   }
-  // warp-reduce the per-thread counters, then one atomic per warp
-  unsigned long long ev = cnt.events, st = cnt.steps, dr = cnt.draws;
-  for (int o = 16; o > 0; o >>= 1) {
-    ev += __shfl_down_sync(kFull, ev, o);
-    st += __shfl_down_sync(kFull, st, o);
-    dr += __shfl_down_sync(kFull, dr, o);
-  }
-  if (lane == 0) {
-    atomicAdd(&rp.scratch->events, ev);
-    atomicAdd(&rp.scratch->steps, st);
-    atomicAdd(&rp.scratch->draws, dr);
+  if constexpr (kCount) {      // warp-reduce the per-thread counters, then one atomic per warp
+    unsigned long long ev = cnt.events, st = cnt.steps, dr = cnt.draws;
+    for (int o = 16; o > 0; o >>= 1) {
+      ev += __shfl_down_sync(kFull, ev, o);
+      st += __shfl_down_sync(kFull, st, o);
+      dr += __shfl_down_sync(kFull, dr, o);
+    }
+    if (lane == 0) {
+      atomicAdd(&rp.scratch->events, ev);
+      atomicAdd(&rp.scratch->steps, st);
+      atomicAdd(&rp.scratch->draws, dr);
+    }
   }
   __syncthreads();
   if (threadIdx.x < LMC_MAX_SENSORS && s_hits[threadIdx.x])
     atomicAdd(&rp.scratch->hits[threadIdx.x], s_hits[threadIdx.x]);
+  if (!kCount && threadIdx.x == 0) {   // a flight without an event ended its photon
+    const unsigned long long ev = wide(s_events);
+    atomicAdd(&rp.scratch->events, ev);
+    atomicAdd(&rp.scratch->steps,
+              ev + s_fate[kDetected] + s_fate[kEscaped] + s_fate[kStack] + s_fate[kError]);
+    atomicAdd(&rp.scratch->draws, wide(s_draws));
+  }
   if (threadIdx.x == kError && s_fate[kError])
-    atomicAdd(&rp.scratch->photons, s_fate[kError]);
+    atomicAdd(&rp.scratch->photons, (unsigned long long)s_fate[kError]);
   if (threadIdx.x >= 1 && threadIdx.x < 6 && s_fate[threadIdx.x]) {
     unsigned long long *dst = threadIdx.x == kDetected ? &rp.scratch->detected
                               : threadIdx.x == kEscaped ? &rp.scratch->escaped
                               : threadIdx.x == kStack   ? &rp.scratch->stack
                               : threadIdx.x == kRoulette ? &rp.scratch->roulette
                                                          : &rp.scratch->cap;
-    atomicAdd(dst, s_fate[threadIdx.x]);
-    atomicAdd(&rp.scratch->photons, s_fate[threadIdx.x]);
+    atomicAdd(dst, (unsigned long long)s_fate[threadIdx.x]);
+    atomicAdd(&rp.scratch->photons, (unsigned long long)s_fate[threadIdx.x]);
   }
   if (kEst && rp.est_smem_doubles > 0) {      // the block's estimated grids into the tallies
     const Scene &sc = *scp;
@@ -2714,7 +2768,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2)
   ph.rng.ring = &side.ring[0][threadIdx.x];
   Flight<R> fl;
   fl.score = nullptr;
-  Counters cnt = {0, 0, 0};
+  Counters<false> cnt;
   R *r = static_cast<R *>(q.r);
   const Scene *scp = kSweep ? g_scene : reinterpret_cast<const Scene *>(s_raw);
   unsigned long long slot = 0;

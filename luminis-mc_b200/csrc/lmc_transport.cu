@@ -957,6 +957,16 @@ static lmc_status sweep_adjoint_layout(const lmc_handle *h, const lmc_adjoint_op
 
 }  // extern "C"
 
+static void set_seed(lmc::dev::RunParams &rp, uint64_t seed)
+{
+  rp.key0 = (uint32_t)seed;
+  rp.key1 = (uint32_t)(seed >> 32);
+  for (uint32_t r = 0; r < 10; ++r) {
+    rp.round_key[2 * r] = rp.key0 + r * lmc::dev::kPhiloxStep0;
+    rp.round_key[2 * r + 1] = rp.key1 + r * lmc::dev::kPhiloxStep1;
+  }
+}
+
 // The transport and tally kernels of a run.  `extras`: a scene has a MixtureLayer or an
 // Absorption recorder (the variants with their code; the others leave it out).
 using KernelFn = void (*)(const lmc::dev::Scene *, lmc::dev::RunParams);
@@ -1162,8 +1172,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
                              sizeof(unsigned long long) * h->n_scenes * LMC_MAX_SENSORS, stream));
   dev::RunParams rp;
   std::memset(&rp, 0, sizeof(rp));
-  rp.key0 = (uint32_t)seed;
-  rp.key1 = (uint32_t)(seed >> 32);
+  set_seed(rp, seed);
   rp.max_events = opts->max_events;
   rp.track_reverse = opts->track_reverse_paths ? 1 : 0;
   rp.tallies = d_tallies;
@@ -2147,8 +2156,7 @@ extern "C" lmc_status lmc_run_noalloc(const lmc_scene *s, uint64_t seed, uint64_
   // ---- launches: the same kernels and batch loop as lmc_run, queue in the array
   dev::RunParams rp;
   std::memset(&rp, 0, sizeof(rp));
-  rp.key0 = (uint32_t)seed;
-  rp.key1 = (uint32_t)(seed >> 32);
+  set_seed(rp, seed);
   rp.max_events = opts->max_events;
   rp.track_reverse = opts->track_reverse_paths ? 1 : 0;
   rp.tallies = d_tallies;

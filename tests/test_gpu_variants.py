@@ -63,5 +63,7 @@ def test_variants_without_history_equal_the_general_ones(make, precision, cuda):
     spec = make(12_001)
     default = run_tallies(spec, precision)
     assert default[0]["events"] > 0
-    for options in ({"stage_tables": True}, {"no_replay": True, "stage_tables": True}):
+    # (two blocks per SM: the kernels that count events per thread, not per block)
+    for options in ({"stage_tables": True}, {"no_replay": True, "stage_tables": True},
+                    {"blocks_per_sm": 2}, {"blocks_per_sm": 2, "no_replay": True}):
         assert_same_run(run_tallies(spec, precision, **options), default, TOL[precision])
