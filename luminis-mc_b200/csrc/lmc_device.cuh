@@ -211,6 +211,12 @@ struct RunParams {
   lmc_record *records;                   // this launch's photons: photon_begin + i at records[i]
   Scratch *scratch;
   Queue queue;                           // used by the queued kernel pair
+  // kHitsBuffer: buffer_entries of the queue for every warp, one warp after another (the
+  // fields before kQR1 only); list_cap entries of replay_list for the photons (from
+  // photon_begin) whose CBS hits the rerun launch processes, with sensor_mask's sensors
+  unsigned long long buffer_entries, list_cap;
+  unsigned int sensor_mask;
+  int rerun;
   unsigned int cbs_mask;                 // sensors whose hits need the CBS fields
   unsigned int pad;
   // likelihood-ratio outputs: (1 + adj_K) rows of adj_n_out doubles; row 0 the

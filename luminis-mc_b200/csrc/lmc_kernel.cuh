@@ -842,6 +842,14 @@ __device__ void reverse_field(const Scene &sc, const HitData<R> &h, Cx<R> &Om, C
 // shared-memory grids for the sensors the run privatises.
 constexpr int kTallyGlobal = 0, kTallyWarp = 1, kTallyShared = 2;
 
+// Im(a conj(b)) rounded as the on-the-spot process_hit rounds it in binary32 (a.im b.re fused),
+// so that a scene's tallies do not depend on whether its hits were buffered.
+__device__ __forceinline__ float minus_cross(Cx<float> a, Cx<float> b)
+{
+  return __fmaf_rn(a.im, b.re, -__fmul_rn(a.re, b.im));
+}
+__device__ __forceinline__ double minus_cross(Cx<double> a, Cx<double> b) { return a.im * b.re - a.re * b.im; }
+
 // The four Stokes values of one cell: planes base, base + stride, ... at `off`.
 // kTallyWarp: the lanes of the warp that reach this call together group by cell
 // (__match_any_sync on the address); the lowest lane of each group pulls its peers'
@@ -958,7 +966,7 @@ __device__ __forceinline__ void adj_add_radial(const AdjView &A, double *s_rad, 
 // FarFieldCBSSensor::process_hit (src/detector.cpp:1231-1310) and the far-field
 // fluence sensor (same binning, reverse field zero).  exp(i k L) multiplies E_f
 // and E_r alike and cancels in every Stokes parameter, so it is not formed.
-template <typename R, bool kAdj, int kT = kTallyGlobal>
+template <typename R, bool kAdj, int kT = kTallyGlobal, bool kCbs = true>
 __device__ bool hit_farfield(const Scene &sc, const RunParams &rp, const Sensor &s,
                              const HitData<R> &h, lmc_record *rec, int si, const R *hs, const AdjView *A,
                              double *priv = nullptr)
@@ -987,10 +995,10 @@ __device__ bool hit_farfield(const Scene &sc, const RunParams &rp, const Sensor 
   const unsigned long long P = s.plane_stride;
   if (!in_bounds(kBoundFarfield, (unsigned long long)t_idx * tstride + cell < P))
     return false;
-  if (s.kind == LMC_SENSOR_FARFIELD_FLUENCE) {
+  if (!kCbs || s.kind == LMC_SENSOR_FARFIELD_FLUENCE) {
     const double q0 = (double)(cnorm(Efx) + cnorm(Efy)), q1 = (double)(cnorm(Efx) - cnorm(Efy));
     const Cx<R> xy = cmul(Efx, Cx<R>{Efy.re, -Efy.im});
-    const double q2 = 2.0 * (double)xy.re, q3 = 2.0 * (double)xy.im;
+    const double q2 = 2.0 * (double)xy.re, q3 = 2.0 * (double)(kCbs ? xy.im : minus_cross(Efx, Efy));
     add4<kT>(base, P, cell, q0, q1, q2, q3);
     if (t_idx >= 1)
       add4<kT>(base, P, t_idx * tstride + cell, q0, q1, q2, q3);
@@ -1061,7 +1069,7 @@ __device__ bool hit_farfield(const Scene &sc, const RunParams &rp, const Sensor 
 
 // PlanarFluenceSensor::process_hit (src/detector.cpp:780-841): lab-frame Stokes
 // with E_x negated; exp(i k L) cancels and is not formed.
-template <typename R, bool kAdj, int kT = kTallyGlobal>
+template <typename R, bool kAdj, int kT = kTallyGlobal, bool kSpot = false>
 __device__ bool hit_fluence(const Scene &sc, const RunParams &rp, const Sensor &s, const HitData<R> &h,
                             int si, const R *hs, double *s_rad, const AdjView *A, double *priv = nullptr)
 {
@@ -1084,7 +1092,7 @@ __device__ bool hit_fluence(const Scene &sc, const RunParams &rp, const Sensor &
   const Cx<R> Ey = cadd(cscale(Em, h.P[1]), cscale(En, h.P[4]));
   const Cx<R> xy = cmul(Ex, Cx<R>{Ey.re, -Ey.im});
   const double q0 = (double)(cnorm(Ex) + cnorm(Ey)), q1 = (double)(cnorm(Ex) - cnorm(Ey));
-  const double q2 = 2.0 * (double)xy.re, q3 = 2.0 * (double)xy.im;
+  const double q2 = 2.0 * (double)xy.re, q3 = 2.0 * (double)(kSpot ? minus_cross(Ex, Ey) : xy.im);
   double *base = tally_base<kT>(rp, s, si, priv);
   const unsigned long long cell = (unsigned long long)xi * s.N_y + yi;
   const unsigned long long tstride = (unsigned long long)s.N_x * s.N_y;
@@ -1194,7 +1202,8 @@ __device__ __noinline__ void hit_statistics(const Sensor &s, double *tallies, do
 // process_hit of every sensor in `mask` (all on the plane of this hit), in
 // insertion order, as SensorsGroup::record_hit calls them (src/detector.cpp:244-265).
 // kT: the tally kernel's mode (kTallyShared: priv is the block's private grid area).
-template <typename R, bool kAdj, int kT = kTallyGlobal>
+// kCbs = false: buffered hits, without FarFieldCBS sensors.
+template <typename R, bool kAdj, int kT = kTallyGlobal, bool kCbs = true>
 __device__ void process_hits(const Scene &sc, const RunParams &rp, const HitData<R> &h,
                              unsigned mask, unsigned long long *hits, const R *hs, double *s_rad,
                              const AdjView *A, double *priv = nullptr)
@@ -1208,7 +1217,7 @@ __device__ void process_hits(const Scene &sc, const RunParams &rp, const HitData
     const Sensor &s = sc.sensors[si];
     bool counted;
     if (s.kind == LMC_SENSOR_PLANAR_FLUENCE)
-      counted = hit_fluence<R, kAdj, kT>(sc, rp, s, h, si, hs, s_rad, A, priv);
+      counted = hit_fluence<R, kAdj, kT, !kCbs>(sc, rp, s, h, si, hs, s_rad, A, priv);
     else if (s.kind == LMC_SENSOR_PLANAR_FIELD)
       counted = hit_field<R>(sc, rp, s, h);
     else if (s.kind == LMC_SENSOR_STATISTICS) {
@@ -1220,7 +1229,7 @@ __device__ void process_hits(const Scene &sc, const RunParams &rp, const HitData
       counted = true;
     }
     else
-      counted = hit_farfield<R, kAdj, kT>(sc, rp, s, h, rec, si, hs, A, priv);
+      counted = hit_farfield<R, kAdj, kT, kCbs>(sc, rp, s, h, rec, si, hs, A, priv);
     if (counted && rec) {
       rec->hit[0] = h.hx;
       rec->hit[1] = h.hy;
@@ -1919,16 +1928,13 @@ __device__ __forceinline__ void fill_hit(const Photon<R> &ph, const Side<R> &sid
     h.T[q] = {side.T[2 * q][tid], side.T[2 * q + 1][tid]};
 }
 
-// Whether a hit's FarFieldCBS sensors will read its reverse-path fields: from the
-// second scattering event on (src/detector.cpp:1290) and when the exit direction falls
-// in one of their grids (the binning of hit_farfield, src/detector.cpp:1271-1281),
-// widened by a bin on every side so that no hit a grid bins is missed.
+// Whether a hit's exit direction falls in the grid of one of its FarFieldCBS sensors (the
+// binning of hit_farfield, src/detector.cpp:1271-1281), widened by a bin on every side so
+// that no hit a grid bins is missed.
 template <typename R>
-__device__ __forceinline__ bool needs_reverse(const Scene &sc, unsigned mask, const Photon<R> &ph)
+__device__ __forceinline__ bool sees_cbs_grid(const Scene &sc, unsigned mask, const Photon<R> &ph)
 {
   const unsigned m = mask & sc.cbs_mask;
-  if (!m || ph.events < 2)
-    return false;
   const R theta = exit_theta(ph.P[6], ph.P[7], ph.P[8]);
   R phi = m_atan2(ph.P[7], ph.P[6]);
   if (phi < R(0))
@@ -1944,22 +1950,56 @@ __device__ __forceinline__ bool needs_reverse(const Scene &sc, unsigned mask, co
   return false;
 }
 
-// Append a hit to the queue (warp-aggregated slot).  Only the fields the
-// sensors in `mask` read are written.
-template <typename R, bool kAdj, bool kTrack>
+// The warp's number in its launch.
+__device__ __forceinline__ unsigned long long warp_index()
+{
+  return (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+}
+
+// Whether a hit's FarFieldCBS sensors will read its reverse-path fields: from the second
+// scattering event on (src/detector.cpp:1290), in one of their grids.
+template <typename R>
+__device__ __forceinline__ bool needs_reverse(const Scene &sc, unsigned mask, const Photon<R> &ph)
+{
+  return (mask & sc.cbs_mask) && ph.events >= 2 && sees_cbs_grid<R>(sc, mask, ph);
+}
+
+// Where a launch's hits go: processed on the spot (scenes with planes inside the sample:
+// records, and the rerun of CBS hits); appended to the run's queue for the tally kernel
+// (every plane at z <= 0); or to the warp's own buffer (planes inside the sample, see
+// drain_hits), except for those of FarFieldCBS sensors, whose photons are listed to be run
+// again on the spot with their history.
+constexpr int kHitsInline = 0, kHitsQueue = 1, kHitsBuffer = 2;
+
+// Entries of a warp's hit buffer: fewer than 32 are left by the last drain, and an event
+// adds at most two per lane and plane (a straight flight crosses a plane once; one that
+// lies on an interface can end one segment and start the next).
+__host__ __device__ constexpr unsigned hit_buffer_entries(int n_planes) { return 32 + 64 * n_planes; }
+
+// Append a hit to the queue (warp-aggregated slot) or (kBuffer) to the warp's buffer, whose
+// fill is
+// *fill.  Only the fields the sensors in `mask` read are written.
+template <typename R, bool kAdj, bool kTrack, bool kBuffer>
 __device__ __forceinline__ void enqueue_hit(const Scene &sc, const RunParams &rp, const Photon<R> &ph,
                                             const Side<R> &side, const Flight<R> &fl, R t,
-                                            R hx, R hy, R hz, double opath, unsigned mask)
+                                            R hx, R hy, R hz, double opath, unsigned mask,
+                                            unsigned *fill)
 {
-  const unsigned active = __activemask();
-  const unsigned lane = threadIdx.x & 31u;
-  const int leader = __ffs(active) - 1;
-  unsigned long long base = 0;
-  if ((int)lane == leader)
-    base = atomicAdd(&rp.scratch->queue_count, (unsigned long long)__popc(active));
-  base = __shfl_sync(active, base, leader);
-  const unsigned long long slot = base + __popc(active & ((1u << lane) - 1u));
   const Queue &q = rp.queue;
+  unsigned long long slot;
+  if constexpr (kBuffer) {
+    const unsigned e = atomicAdd(fill, 1u);
+    slot = e < rp.buffer_entries ? warp_index() * rp.buffer_entries + e : q.cap;
+  } else {
+    const unsigned active = __activemask();
+    const unsigned lane = threadIdx.x & 31u;
+    const int leader = __ffs(active) - 1;
+    unsigned long long base = 0;
+    if ((int)lane == leader)
+      base = atomicAdd(&rp.scratch->queue_count, (unsigned long long)__popc(active));
+    base = __shfl_sync(active, base, leader);
+    slot = base + __popc(active & ((1u << lane) - 1u));
+  }
   if (slot >= q.cap) {
     atomicOr(&rp.scratch->error_flags, (unsigned)kErrQueueOverflow);
     return;
@@ -1988,7 +2028,9 @@ __device__ __forceinline__ void enqueue_hit(const Scene &sc, const RunParams &rp
   r[(kQE + 1) * C + slot] = ph.Em.im;
   r[(kQE + 2) * C + slot] = ph.En.re;
   r[(kQE + 3) * C + slot] = ph.En.im;
-  if ((mask & sc.cbs_mask) && (!kTrack || rp.cbs_replay)) {
+  if constexpr (kBuffer) {
+    return;                              // no CBS hits here
+  } else if ((mask & sc.cbs_mask) && (!kTrack || rp.cbs_replay)) {
     // no history kept: the replay kernel rebuilds it for the hits a grid will read
     if (needs_reverse<R>(sc, mask, ph)) {
       const unsigned long long k = atomicAdd(&rp.scratch->replay_count, 1ull);
@@ -2019,13 +2061,102 @@ __device__ __forceinline__ void enqueue_hit(const Scene &sc, const RunParams &rp
       r[(kQScore + k) * C + slot] = flight_hit_score<R>(sc, fl, t, k);
 }
 
+// Hit-queue entry i; returns its sensor mask.  kCbs = false: an entry of a warp's buffer.
+template <typename R, bool kCbs = true>
+__device__ __forceinline__ unsigned load_hit(const Scene &sc, const Queue &q, unsigned long long i,
+                                             HitData<R> &h)
+{
+  const unsigned long long C = q.cap;
+  const R *r = static_cast<const R *>(q.r);
+  h.p_lo = q.u32[kQPhotonLo * C + i];
+  h.p_hi = q.u32[kQPhotonHi * C + i];
+  h.events = q.u32[kQEvents * C + i];
+  const unsigned mask = q.u32[kQMask * C + i];
+  const uint32_t media = q.u32[kQMedia * C + i];
+  h.first_med = media & 0xffffu;
+  h.last_med = media >> 16;
+  h.w = q.f64[kQWeight * C + i];
+  h.opath = q.f64[kQOpath * C + i];
+  h.pen = (mask & sc.stat_mask) ? q.f64[kQPen * C + i] : 0.0;
+  h.hx = r[(kQHit + 0) * C + i];
+  h.hy = r[(kQHit + 1) * C + i];
+  h.hz = r[(kQHit + 2) * C + i];
+#pragma unroll
+  for (int j = 0; j < 9; ++j)
+    h.P[j] = r[(kQP + j) * C + i];
+  h.Em = {r[(kQE + 0) * C + i], r[(kQE + 1) * C + i]};
+  h.En = {r[(kQE + 2) * C + i], r[(kQE + 3) * C + i]};
+  if (kCbs && (mask & sc.cbs_mask)) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      h.r1[j] = r[(kQR1 + j) * C + i];
+      h.rn[j] = r[(kQRn + j) * C + i];
+    }
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      h.P1[j] = r[(kQP1 + j) * C + i];
+      h.Pn1[j] = r[(kQPn1 + j) * C + i];
+    }
+#pragma unroll
+    for (int qd = 0; qd < 4; ++qd)
+      h.T[qd] = {r[(kQT + 2 * qd) * C + i], r[(kQT + 2 * qd + 1) * C + i]};
+  }
+  return mask;
+}
+
+// The warp's buffered hits [first, first + n), n <= 32, one a lane: process_hit of their
+// sensors.  Sensor planes inside the sample are crossed any number of times, so no queue
+// bounds their hits; on the spot they ran with the one or two lanes that crossed, at
+// nearly every event, and their code took the transport to 237 registers (one block per
+// SM).  Collected per warp they run 32 at a time, out of line, so that the transport keeps
+// the registers its events need.  1 M bilayer photons with three fluence planes and a
+// statistics plane inside and the cone at the surface: 44.0 -> 22.9 ms (one
+// fluence plane alone: 26.8 -> 12.0; binary64, 0.3 M photons: 30.0 -> 18.8).
+template <typename R>
+__device__ __noinline__ void drain_hits(const Scene &sc, const RunParams &rp, unsigned long long first,
+                                        unsigned n, unsigned long long *s_hits)
+{
+  const unsigned lane = threadIdx.x & 31u;
+  __syncwarp();                          // the entries, written by other lanes
+  if (lane < n) {
+    HitData<R> h;
+    const unsigned mask = load_hit<R, false>(sc, rp.queue, first + lane, h);
+    process_hits<R, false, kTallyGlobal, false>(sc, rp, h, mask, s_hits, nullptr, nullptr, nullptr);
+  }
+  __syncwarp();                          // read before their slots are written again
+}
+
+// Words of a thread's state that go through local memory around drain_hits: held in
+// registers across the call they would be spilled in the event loop instead.
+template <typename T> struct Parked {
+  static constexpr int kWords = sizeof(T) / 4;
+  static_assert(sizeof(T) % 4 == 0, "whole words");
+  volatile uint32_t w[kWords];
+  __device__ __forceinline__ void put(const T &v)
+  {
+    uint32_t u[kWords];
+    memcpy(u, &v, sizeof(T));
+#pragma unroll
+    for (int j = 0; j < kWords; ++j)
+      w[j] = u[j];
+  }
+  __device__ __forceinline__ void get(T &v) const
+  {
+    uint32_t u[kWords];
+#pragma unroll
+    for (int j = 0; j < kWords; ++j)
+      u[j] = w[j];
+    memcpy(&v, u, sizeof(T));
+  }
+};
+
 // SensorsGroup::record_hit (src/detector.cpp:178-270) for the step (x0,y0,z0) -> pos.
-// kQueue: hits are appended to the queue for the tally kernel; otherwise they are
-// processed here.  Returns whether an absorbing sensor took the photon.
-template <typename R, bool kQueue, bool kAdj, bool kTrack = true>
+// kHitsTo: hits are processed here, or appended to the queue or to the warp's buffer.
+// Returns whether an absorbing sensor took the photon.
+template <typename R, int kHitsTo, bool kAdj, bool kTrack = true>
 __device__ __forceinline__ bool record_hit(const Scene &sc, const RunParams &rp, Photon<R> &ph,
                                            const Side<R> &side, const Flight<R> &fl, R x0, R y0, R z0,
-                                           unsigned long long *s_hits)
+                                           unsigned long long *s_hits, unsigned *fill)
 {
   const R z1 = z0, z2 = ph.pz;
   const int crossing = (z2 > z1) ? 0 : 1;
@@ -2053,9 +2184,18 @@ __device__ __forceinline__ bool record_hit(const Scene &sc, const RunParams &rp,
         killed = true;
     }
     if (mask) {
-      if (kQueue) {
-        enqueue_hit<R, kAdj, kTrack>(sc, rp, ph, side, fl, t, hx, hy, hz, opath, mask);
-      } else {
+      if constexpr (kHitsTo == kHitsBuffer) {
+        if ((mask & sc.cbs_mask) && sees_cbs_grid<R>(sc, mask, ph)) {
+          const unsigned long long k = atomicAdd(&rp.scratch->replay_count, 1ull);
+          if (k < rp.list_cap)
+            rp.replay_list[k] = (uint32_t)(ph.index() - rp.photon_begin);
+        }
+        mask &= ~sc.cbs_mask;
+        if (mask)
+          enqueue_hit<R, kAdj, kTrack, true>(sc, rp, ph, side, fl, t, hx, hy, hz, opath, mask, fill);
+      } else if constexpr (kHitsTo == kHitsQueue) {
+        enqueue_hit<R, kAdj, kTrack, false>(sc, rp, ph, side, fl, t, hx, hy, hz, opath, mask, fill);
+      } else if ((mask &= rp.sensor_mask) != 0u) {
         HitData<R> h;
         fill_hit<R>(ph, side, hx, hy, hz, opath, h);
         process_hits<R, false>(sc, rp, h, mask, s_hits, nullptr, nullptr, nullptr);
@@ -2177,12 +2317,12 @@ __device__ __forceinline__ void record_absorption_f32(const AbsorbGrid &g, doubl
 // (scenes without either run the variant without their code).  kHits = false (the CBS
 // replay) leaves the sensor planes out: a replayed event never reaches one, because
 // crossing a plane at z <= 0 ends a photon.  kTrack = false (see transport_kernel) leaves
-// the reverse-path history and, without kExtras, the penetration depth out.
-template <typename R, bool kQueue, bool kAdj, bool kExtras = false, bool kHits = true, bool kTrack = true,
+// the reverse-path history and, of queued launches without kExtras, the penetration depth out.
+template <typename R, int kHitsTo, bool kAdj, bool kExtras = false, bool kHits = true, bool kTrack = true,
           bool kKeys = false, bool kCount = true>
 __device__ __forceinline__ int event_move(const Scene &sc, const RunParams &rp, Photon<R> &ph,
                                           Side<R> &side, Flight<R> &fl, Counters<kCount> &cnt,
-                                          unsigned long long *s_hits, int &med_out)
+                                          unsigned long long *s_hits, int &med_out, unsigned *fill = nullptr)
 {
   rng_prefetch<R, kKeys>(ph.rng, rp);
   {
@@ -2219,7 +2359,7 @@ __device__ __forceinline__ int event_move(const Scene &sc, const RunParams &rp, 
         ph.pz = m_nudge(zi + ((dz > R(0)) ? R(1e-12) : R(-1e-12)), zi, dz > R(0));
       } else {
         ph.pz += dz * s_move;
-        if ((kTrack || kExtras) && ph.pz > ph.pen)
+        if ((kTrack || kExtras || kHitsTo == kHitsBuffer) && ph.pz > ph.pen)
           ph.pen = ph.pz;
       }
       if (kAdj) {
@@ -2229,7 +2369,7 @@ __device__ __forceinline__ int event_move(const Scene &sc, const RunParams &rp, 
       if (kHits && sc.n_planes > 0 && fabs(ph.pz - z0) >= R(1e-12)) {
         const R zlo = z0 < ph.pz ? z0 : ph.pz, zhi = z0 < ph.pz ? ph.pz : z0;
         if (sc_plane<R>(sc, 0) <= zhi && sc_plane<R>(sc, sc.n_planes - 1) >= zlo &&
-            record_hit<R, kQueue, kAdj, kTrack>(sc, rp, ph, side, fl, x0, y0, z0, s_hits))
+            record_hit<R, kHitsTo, kAdj, kTrack>(sc, rp, ph, side, fl, x0, y0, z0, s_hits, fill))
           return kDetected;
       }
       if (!at_iface)
@@ -2434,7 +2574,7 @@ __device__ __forceinline__ int event_scatter(const Scene &sc, const RunParams &r
   }
   ph.events++;                                                // :578-587
   cnt.event();
-  if (kExtras && kDeposit && (lflags & kLayerAbsorb)) {       // :589-592
+  if (kExtras && kDeposit && (lflags & kLayerAbsorb) && !rp.rerun) {   // :589-592
     const double t = sc.absorb.d_t > 0.0 ? launch_time<R>(sc, rp, ph) + ph.opath : 0.0;  // velocity 1
     const double dw = SL.mu_t > 0 ? ph.w * SL.absorb_prob : 1.0;
     if constexpr (std::is_same<R, float>::value)
@@ -2456,15 +2596,15 @@ __device__ __forceinline__ int event_scatter(const Scene &sc, const RunParams &r
 
 // One loop iteration of run_photon (src/simulation.cpp:297-614).  Returns the photon's
 // fate (kAlive if it continues).
-template <typename R, bool kQueue, bool kAdj, bool kExtras = false, bool kTrack = true, bool kStaged = true,
+template <typename R, int kHitsTo, bool kAdj, bool kExtras = false, bool kTrack = true, bool kStaged = true,
           bool kKeys = false, bool kCount = true>
 __device__ __forceinline__ int event_step(const Scene &sc, const RunParams &rp, Photon<R> &ph,
                                           Side<R> &side, Flight<R> &fl, Counters<kCount> &cnt,
-                                          unsigned long long *s_hits)
+                                          unsigned long long *s_hits, unsigned *fill)
 {
   int med_idx = 0;
   const int fate =
-      event_move<R, kQueue, kAdj, kExtras, true, kTrack, kKeys>(sc, rp, ph, side, fl, cnt, s_hits, med_idx);
+      event_move<R, kHitsTo, kAdj, kExtras, true, kTrack, kKeys>(sc, rp, ph, side, fl, cnt, s_hits, med_idx, fill);
   if (fate != kAlive)
     return fate;
   return event_scatter<R, kAdj, kExtras, true, kTrack, kStaged, kKeys>(sc, rp, ph, side, fl, cnt, med_idx);
@@ -2579,14 +2719,15 @@ __device__ __forceinline__ int sweep_scene(const RunParams &rp, unsigned long lo
 // (every flight ends in an event or in one of the fates below): three registers fewer over
 // the loop, spills 48 -> 10 bytes, 20 M bilayer photons 179.5 -> 170.4 ms.  Kernels with
 // registers to spare lose 1-3 % to the adds and count per thread.
-template <typename R, bool kQueue, int kMinBlocks, bool kAdj = false, bool kSweep = false, bool kEst = false,
+template <typename R, int kHitsTo, int kMinBlocks, bool kAdj = false, bool kSweep = false, bool kEst = false,
           bool kExtras = false, bool kTrack = true>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Scene *__restrict__ g_scene, RunParams rp)
+__global__ void __launch_bounds__(kBlock, kMinBlocks)
+    transport_kernel(const Scene *__restrict__ g_scene, const __grid_constant__ RunParams rp)
 {
   __shared__ __align__(16) unsigned char s_raw[kSweep ? 16 : sizeof(Scene)];
   __shared__ unsigned long long s_hits[LMC_MAX_SENSORS];
   // a queued launch's photons fit its queue (fewer than 2^32); an inline launch has no bound
-  using Fates = std::conditional_t<kQueue, unsigned, unsigned long long>;
+  using Fates = std::conditional_t<kHitsTo == kHitsQueue, unsigned, unsigned long long>;
   __shared__ Fates s_fate[7];
   __shared__ unsigned s_events[2], s_draws[2];
   constexpr bool kCount = kMinBlocks < 4;
@@ -2618,24 +2759,42 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
   Counters<kCount> cnt;
   Photon<R> ph;
   ph.rng.ring = &side.ring[0][threadIdx.x];
+  // kHitsInline: the photons of the replay list instead (rp.rerun), for their CBS hits
+  const bool listed = kHitsTo == kHitsInline && rp.rerun;
+  unsigned long long n_run = rp.n_photons;
+  if (listed) {
+    const unsigned long long c = *(volatile unsigned long long *)&rp.scratch->replay_count;
+    n_run = c < rp.list_cap ? c : rp.list_cap;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      atomicAdd(&rp.scratch->replayed, n_run);
+  }
+  unsigned long long *const next = listed ? &rp.scratch->replay_next : &rp.scratch->next_photon;
   bool alive = false, done = false;
+  __shared__ unsigned s_fill[kBlock / 32];     // kHitsBuffer: hits in each warp's buffer
+  unsigned *const fill = s_fill + (threadIdx.x >> 5);
+  if (kHitsTo == kHitsBuffer) {
+    if (lane == 0)
+      *fill = 0;
+    __syncwarp();
+  }
   for (;;) {
     const unsigned need = __ballot_sync(kFull, !alive && !done);
     if (need) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
       if ((int)lane == leader)
-        base = atomicAdd(&rp.scratch->next_photon, (unsigned long long)__popc(need));
+        base = atomicAdd(next, (unsigned long long)__popc(need));
       base = __shfl_sync(kFull, base, leader);
       if (!alive && !done) {
         const unsigned long long idx = base + __popc(need & ((1u << lane) - 1u));
-        if (idx < rp.n_photons) {
+        if (idx < n_run) {
+          const unsigned long long at = rp.photon_begin + (listed ? rp.replay_list[idx] : idx);
           int si = 0;
           if (kSweep) {
-            si = sweep_scene(rp, rp.photon_begin + idx);
+            si = sweep_scene(rp, at);
             scp = g_scene + si;
           }
-          init_photon<R, kTrack>(*scp, rp, ph, side, rp.photon_begin + idx);
+          init_photon<R, kTrack>(*scp, rp, ph, side, at);
           ph.scene = si;
           if (kAdj)
             for (int k = 0; k < rp.adj_K; ++k)
@@ -2646,7 +2805,28 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
         }
       }
     }
-    if (__all_sync(kFull, done))
+    const bool finished = __all_sync(kFull, done);
+    if constexpr (kHitsTo == kHitsBuffer) {
+      // full groups of 32 hits, all of them when the warp is done
+      __syncwarp();
+      unsigned n = *(volatile unsigned *)fill;
+      if (n >= 32u || (finished && n > 0u)) {
+        Parked<Photon<R>> parked;
+        parked.put(ph);
+        const unsigned long long first = warp_index() * rp.buffer_entries;
+        while (n >= 32u || (finished && n > 0u)) {
+          const unsigned m = n < 32u ? n : 32u;
+          n -= m;
+          drain_hits<R>(*scp, rp, first + n, m, s_hits);
+        }
+        parked.get(ph);
+        ph.rng.ring = &side.ring[0][threadIdx.x];    // shared memory, known to be so
+        if (lane == 0)
+          *fill = n;
+        __syncwarp();
+      }
+    }
+    if (finished)
       break;
     int fate = kAlive;
     if constexpr (kEst) {
@@ -2654,12 +2834,13 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
       // then the scatter
       int med_idx = 0;
       if (alive)
-        fate = event_move<R, kQueue, kAdj, kExtras, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, s_hits, med_idx);
+        fate = event_move<R, kHitsTo, kAdj, kExtras, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, s_hits, med_idx);
       estimate_warp<R>(*scp, rp, ph, side, med_idx, alive && fate == kAlive, s_hits, s_est);
       if (alive && fate == kAlive)
         fate = event_scatter<R, kAdj, kExtras, true, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, med_idx);
     } else if (alive) {
-      fate = event_step<R, kQueue, kAdj, kExtras, kTrack, kTrack && !kSweep, kKeys>(*scp, rp, ph, side, fl, cnt, s_hits);
+      fate = event_step<R, kHitsTo, kAdj, kExtras, kTrack, kTrack && !kSweep, kKeys>(*scp, rp, ph, side, fl, cnt,
+                                                                                   s_hits, fill);
     }
     if (alive) {
       if (fate != kAlive) {
@@ -2687,7 +2868,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
       st += __shfl_down_sync(kFull, st, o);
       dr += __shfl_down_sync(kFull, dr, o);
     }
-    if (lane == 0) {
+    if (lane == 0 && !listed) {
       atomicAdd(&rp.scratch->events, ev);
       atomicAdd(&rp.scratch->steps, st);
       atomicAdd(&rp.scratch->draws, dr);
@@ -2696,6 +2877,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) transport_kernel(const Sce
   __syncthreads();
   if (threadIdx.x < LMC_MAX_SENSORS && s_hits[threadIdx.x])
     atomicAdd(&rp.scratch->hits[threadIdx.x], s_hits[threadIdx.x]);
+  if (listed)                  // the run's photons were counted by their first launch
+    return;
   if (!kCount && threadIdx.x == 0) {   // a flight without an event ended its photon
     const unsigned long long ev = wide(s_events);
     atomicAdd(&rp.scratch->events, ev);
@@ -2804,7 +2987,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2)
       continue;
     if (ph.events < target) {                    // one more event of this replay
       int med = 0;
-      int fate = event_move<R, true, false, kExtras, false>(*scp, rp, ph, side, fl, cnt, nullptr, med);
+      int fate = event_move<R, kHitsQueue, false, kExtras, false>(*scp, rp, ph, side, fl, cnt, nullptr, med);
       if (fate == kAlive)
         fate = event_scatter<R, false, kExtras, false, true, false>(*scp, rp, ph, side, fl, cnt, med);
       if (fate != kAlive) {                      // ended before its recorded hit
@@ -2892,39 +3075,7 @@ __global__ void __launch_bounds__(kBlock, (sizeof(R) == 4 && !(kAdj && kSweep)) 
     const unsigned scene = kSweep ? q.u32[kQScene * C + i] : 0u;
     const Scene &sc = kSweep ? g_scene[scene] : sc0;
     HitData<R> h;
-    h.p_lo = q.u32[kQPhotonLo * C + i];
-    h.p_hi = q.u32[kQPhotonHi * C + i];
-    h.events = q.u32[kQEvents * C + i];
-    const unsigned mask = q.u32[kQMask * C + i];
-    const uint32_t media = q.u32[kQMedia * C + i];
-    h.first_med = media & 0xffffu;
-    h.last_med = media >> 16;
-    h.w = q.f64[kQWeight * C + i];
-    h.opath = q.f64[kQOpath * C + i];
-    h.pen = (mask & sc.stat_mask) ? q.f64[kQPen * C + i] : 0.0;
-    h.hx = r[(kQHit + 0) * C + i];
-    h.hy = r[(kQHit + 1) * C + i];
-    h.hz = r[(kQHit + 2) * C + i];
-#pragma unroll
-    for (int j = 0; j < 9; ++j)
-      h.P[j] = r[(kQP + j) * C + i];
-    h.Em = {r[(kQE + 0) * C + i], r[(kQE + 1) * C + i]};
-    h.En = {r[(kQE + 2) * C + i], r[(kQE + 3) * C + i]};
-    if (mask & sc.cbs_mask) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        h.r1[j] = r[(kQR1 + j) * C + i];
-        h.rn[j] = r[(kQRn + j) * C + i];
-      }
-#pragma unroll
-      for (int j = 0; j < 9; ++j) {
-        h.P1[j] = r[(kQP1 + j) * C + i];
-        h.Pn1[j] = r[(kQPn1 + j) * C + i];
-      }
-#pragma unroll
-      for (int qd = 0; qd < 4; ++qd)
-        h.T[qd] = {r[(kQT + 2 * qd) * C + i], r[(kQT + 2 * qd + 1) * C + i]};
-    }
+    const unsigned mask = load_hit<R>(sc, q, i, h);
     R hs[kAdj ? kAdjMaxK : 1];
     AdjView A;
     if (kAdj) {

@@ -91,6 +91,7 @@ struct lmc_handle {
   unsigned cbs_mask = 0;                 // sensors that need the CBS fields of a hit
   bool queued = false;                   // every sensor plane at z <= 0: queued kernel pair
   int max_planes = 0;                    // most sensor planes of any scene
+  bool deep_cbs = false;                 // a FarFieldCBS sensor on a plane above z = 0
   bool has_est = false;                  // an estimator-mode FarFieldCBS sensor
   // sweep handles (lmc_create_sweep): n_scenes scenes in one device array
   bool sweep = false;
@@ -795,6 +796,8 @@ lmc_status lmc_create(const lmc_scene *s, lmc_handle **out)
   h->queued = b.queued;
   h->cbs_mask = b.cbs_mask;
   h->max_planes = b.sc.n_planes;
+  for (int i = 0; i < b.sc.n_sensors; ++i)   // (planes within 1e-9 of one another are one)
+    h->deep_cbs |= ((b.sc.cbs_mask >> i) & 1u) && b.sc.plane_z[b.sc.sensors[i].plane] > 0.0;
   h->has_est = b.has_est;
   h->abs_off = b.abs_off;
   h->abs_count = b.abs_count;
@@ -977,40 +980,50 @@ static KernelFn pick_transport_t(bool fp32, bool wide, bool adj, bool sw)
 {
   using namespace lmc::dev;
   if (sw && adj)
-    return fp32 ? transport_kernel<float, true, 3, true, true, false, false, T>
-                : transport_kernel<double, true, 1, true, true, false, false, T>;
+    return fp32 ? transport_kernel<float, kHitsQueue, 3, true, true, false, false, T>
+                : transport_kernel<double, kHitsQueue, 1, true, true, false, false, T>;
   if (sw)
-    return fp32 ? transport_kernel<float, true, 3, false, true, false, E, T>
-                : transport_kernel<double, true, 2, false, true, false, E, T>;
+    return fp32 ? transport_kernel<float, kHitsQueue, 3, false, true, false, E, T>
+                : transport_kernel<double, kHitsQueue, 2, false, true, false, E, T>;
   if (adj)
-    return fp32 ? transport_kernel<float, true, 3, true, false, false, false, T>
-                : transport_kernel<double, true, 1, true, false, false, false, T>;
+    return fp32 ? transport_kernel<float, kHitsQueue, 3, true, false, false, false, T>
+                : transport_kernel<double, kHitsQueue, 1, true, false, false, false, T>;
   if (fp32)
-    return wide ? transport_kernel<float, true, 4, false, false, false, E, T>
-                : transport_kernel<float, true, 2, false, false, false, E, T>;
-  return transport_kernel<double, true, 2, false, false, false, E, T>;
+    return wide ? transport_kernel<float, kHitsQueue, 4, false, false, false, E, T>
+                : transport_kernel<float, kHitsQueue, 2, false, false, false, E, T>;
+  return transport_kernel<double, kHitsQueue, 2, false, false, false, E, T>;
 }
 
 template <bool E>
-static KernelFn pick_transport_e(bool fp32, bool queued, bool wide, bool adj, bool sw, bool est, bool track)
+static KernelFn pick_transport_e(bool fp32, bool queued, bool wide, bool adj, bool sw, bool est, bool track,
+                                 bool buffered)
 {
   using namespace lmc::dev;
   if (est)
-    return fp32 ? transport_kernel<float, true, 2, false, false, true, E>
-                : transport_kernel<double, true, 2, false, false, true, E>;
+    return fp32 ? transport_kernel<float, kHitsQueue, 2, false, false, true, E>
+                : transport_kernel<double, kHitsQueue, 2, false, false, true, E>;
+  if (!queued && !buffered)
+    return fp32 ? transport_kernel<float, kHitsInline, 1, false, false, false, E>
+                : transport_kernel<double, kHitsInline, 1, false, false, false, E>;
+  // binary32 at 4 blocks per SM: 22.9 ms for 1 M photons with 5 planes, 25.2 at 3, 28.8 at 2
+  if (!queued && track)
+    return fp32 ? transport_kernel<float, kHitsBuffer, 4, false, false, false, E>
+                : transport_kernel<double, kHitsBuffer, 2, false, false, false, E>;
   if (!queued)
-    return fp32 ? transport_kernel<float, false, 1, false, false, false, E>
-                : transport_kernel<double, false, 1, false, false, false, E>;
+    return fp32 ? transport_kernel<float, kHitsBuffer, 4, false, false, false, E, false>
+                : transport_kernel<double, kHitsBuffer, 2, false, false, false, E, false>;
   return track ? pick_transport_t<E, true>(fp32, wide, adj, sw)
                : pick_transport_t<E, false>(fp32, wide, adj, sw);
 }
 
 // track: the launch keeps the reverse-path history, stages tables or writes records.
+// buffered (not queued): hits go through the warps' buffers instead of being processed on
+// the spot.
 static KernelFn pick_transport(bool fp32, bool queued, bool wide, bool adj, bool sw, bool est, bool extras,
-                               bool track)
+                               bool track, bool buffered)
 {
-  return extras ? pick_transport_e<true>(fp32, queued, wide, adj, sw, est, track)
-                : pick_transport_e<false>(fp32, queued, wide, adj, sw, est, track);
+  return extras ? pick_transport_e<true>(fp32, queued, wide, adj, sw, est, track, buffered)
+                : pick_transport_e<false>(fp32, queued, wide, adj, sw, est, track, buffered);
 }
 
 template <int kT>
@@ -1291,15 +1304,25 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   const bool replay = h->queued && !est && !opts->records && !opts->no_replay &&
                       opts->track_reverse_paths && any_cbs;
   rp.cbs_replay = replay ? 1 : 0;
-  const bool track = !h->queued || est || opts->records || opts->stage_tables || (any_cbs && !replay);
-  // StatisticsSensors read the penetration depth, which the variants without history carry
-  // beside the extras only
+  // Planes inside the sample: hits go through the warps' buffers, and the photons whose CBS
+  // hits a grid reads are run again with their history.  Records keep a photon's last hit,
+  // which needs its hits in order, and a CBS plane above z = 0 could list a photon twice:
+  // those runs (and no_replay) process every hit on the spot.
+  const bool buffered = !h->queued && !opts->records && !opts->no_replay && !h->deep_cbs &&
+                        h->tally_doubles > 0;
+  const bool rerun = buffered && any_cbs;
+  rp.sensor_mask = ~0u;
+  const bool track = (!h->queued && !buffered) || est || opts->records || opts->stage_tables ||
+                     (any_cbs && !replay && !rerun);
+  // StatisticsSensors read the penetration depth, which the queued variants without history
+  // carry beside the extras only
   bool any_stat = false;
   for (int k = 0; k < h->n_scenes; ++k)
     any_stat = any_stat || (sw ? h->scenes[k] : h->scene).stat_mask != 0;
   const KernelFn tk = pick_transport(fp32, h->queued, wide, adj != nullptr, sw, est,
-                                     extras || (!track && !adj && any_stat), track || (adj && any_stat));
-  if (replay || !track) {                // no history: the ring and first species only
+                                     extras || (!track && !adj && any_stat && h->queued), track || (adj && any_stat),
+                                     buffered);
+  if (replay || !track || rerun) {       // no history: the ring and first species only
     rp.track_reverse = 0;
     dyn_transport = fp32 ? dev::side_slim_bytes<float>() : dev::side_slim_bytes<double>();
   }
@@ -1307,10 +1330,12 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   rp.side_off = (unsigned)dyn_transport;
   if (adj)
     dyn_transport += (size_t)rp.adj_K * dev::kBlock * rbytes;
-  const KernelFn tr = replay ? pick_replay(fp32, sw, extras) : nullptr;
+  const KernelFn tr = replay ? pick_replay(fp32, sw, extras)
+                      : rerun ? pick_transport(fp32, false, false, false, false, false, extras, true, false)
+                              : nullptr;
   const size_t dyn_replay = fp32 ? dev::side_bytes<float>() : dev::side_bytes<double>();
   int replay_grid = 0;
-  if (replay) {
+  if (tr) {
     LMC_CUDA(cudaFuncSetAttribute((const void *)tr, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)dyn_replay));
     int per = 0;
@@ -1373,14 +1398,26 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
 
   // batches: the whole range at once inline; queue-sized batches when queued
   unsigned long long batch = n_photons;
-  if (h->queued && n_photons > 0) {
+  const unsigned long long full_grid = (unsigned long long)h->sm_count * per_sm;
+  if ((h->queued || buffered) && n_photons > 0) {
     batch = opts->batch_photons ? opts->batch_photons : (32ull << 20);   // ~110 B of queue per photon
     batch = std::min<unsigned long long>(batch, n_photons);
-    const unsigned long long planes = std::max(1, h->max_planes);
-    const unsigned long long cap = batch * planes + batch / 16 + 1024;
-    const size_t need = (size_t)cap * (dev::kQU32Fields * 4 + dev::kQF64Fields * 8 +
-                                       (dev::kQRFields + (size_t)rp.adj_K) * rbytes) +
-                        (replay ? (size_t)cap * sizeof(uint32_t) : 0) + 4 * 256;
+    unsigned long long cap;
+    size_t fields = dev::kQRFields + (size_t)rp.adj_K;
+    if (h->queued) {
+      const unsigned long long planes = std::max(1, h->max_planes);
+      cap = batch * planes + batch / 16 + 1024;
+      rp.list_cap = replay ? cap : 0;
+    } else {                             // one buffer per warp of the launch
+      rp.buffer_entries = dev::hit_buffer_entries(h->max_planes);
+      cap = std::min<unsigned long long>(full_grid, (batch + block - 1) / block) * (block / 32) *
+            rp.buffer_entries;
+      fields = dev::kQRBasic;
+      batch = std::min<unsigned long long>(batch, 1ull << 31);   // listed by 32-bit offset
+      rp.list_cap = rerun ? batch : 0;   // a photon leaves through z = 0 once
+    }
+    const size_t need = (size_t)cap * (dev::kQU32Fields * 4 + dev::kQF64Fields * 8 + fields * rbytes) +
+                        (size_t)rp.list_cap * sizeof(uint32_t) + 4 * 256;
     if (h->queue_bytes < need) {
       cudaFree(h->d_queue);
       h->d_queue = nullptr;
@@ -1399,8 +1436,8 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     rp.queue.f64 = reinterpret_cast<double *>(q + o);
     o += align((size_t)cap * dev::kQF64Fields * 8);
     rp.queue.r = q + o;
-    o += align((size_t)cap * (dev::kQRFields + (size_t)rp.adj_K) * rbytes);
-    rp.replay_list = replay ? reinterpret_cast<uint32_t *>(q + o) : nullptr;
+    o += align((size_t)cap * fields * rbytes);
+    rp.replay_list = rp.list_cap ? reinterpret_cast<uint32_t *>(q + o) : nullptr;
   }
   if (stats && n_photons > 0) {           // one event pair per transport launch
     const size_t need_ev = 2 * (size_t)((n_photons + batch - 1) / batch);
@@ -1420,15 +1457,22 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     // reset the work counters (transport, replay) and the queue fills of this batch
     LMC_CUDA(cudaMemsetAsync(h->d_scratch, 0, 4 * sizeof(unsigned long long), stream));
     const int grid = (int)std::max<unsigned long long>(
-        1ull, std::min<unsigned long long>((unsigned long long)h->sm_count * per_sm,
-                                           (nb + block - 1) / block));
+        1ull, std::min<unsigned long long>(full_grid, (nb + block - 1) / block));
     const size_t pair = 2 * (size_t)(done / batch);
     if (stats)
       LMC_CUDA(cudaEventRecord(h->kev[pair], stream));
     tk<<<grid, block, dyn_transport, stream>>>(h->d_scene, rp);
     LMC_CUDA(cudaGetLastError());
-    if (replay) {                        // part of the transport (timed with it)
-      tr<<<replay_grid, dev::kBlock, dyn_replay, stream>>>(h->d_scene, rp);
+    if (tr) {                            // part of the transport (timed with it)
+      dev::RunParams rr = rp;
+      if (rerun) {
+        rr.rerun = 1;
+        rr.track_reverse = 1;
+        rr.side_off = (unsigned)dyn_replay;
+        rr.stage_bytes = 0;
+        rr.sensor_mask = h->scene.cbs_mask;
+      }
+      tr<<<replay_grid, dev::kBlock, dyn_replay, stream>>>(h->d_scene, rr);
       LMC_CUDA(cudaGetLastError());
     }
     if (stats)
@@ -1465,7 +1509,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     }
     stats->transport_ms = (float)tms;
     stats->transport_launches = (uint32_t)launches;
-    stats->replay_launches = replay ? (uint32_t)launches : 0u;
+    stats->replay_launches = tr ? (uint32_t)launches : 0u;
     stats->replayed = sc.replayed;
     if (sc.error_flags)
       return fail(LMC_ERR_KERNEL, "transport kernel raised error flags " + std::to_string(sc.error_flags));
@@ -2162,6 +2206,7 @@ extern "C" lmc_status lmc_run_noalloc(const lmc_scene *s, uint64_t seed, uint64_
   rp.tallies = d_tallies;
   rp.records = static_cast<lmc_record *>(opts->records);
   rp.scratch = d_counters;
+  rp.sensor_mask = ~0u;
   rp.cbs_mask = cbs_mask;
   const bool fp32 = opts->precision == LMC_PRECISION_FP32;
   if (opts->stream_format != 0 && opts->stream_format != 1)
@@ -2172,7 +2217,7 @@ extern "C" lmc_status lmc_run_noalloc(const lmc_scene *s, uint64_t seed, uint64_
     return fail(LMC_ERR_INVALID, "block_size must be a multiple of 32 and at most 256");
   // the kernels lmc_run picks for the same scene and options
   const bool wide = fp32 && queued && (opts->blocks_per_sm == 0 || opts->blocks_per_sm >= 3);
-  const KernelFn tk = pick_transport(fp32, queued, wide, false, false, false, scene_extras(sc), true);
+  const KernelFn tk = pick_transport(fp32, queued, wide, false, false, false, scene_extras(sc), true, false);
   TallyLaunch tl{};
   if (queued && s->n_sensors > 0) {
     const lmc_status st = tally_setup(opts->tally_mode, false, fp32, false, sc, sensor_count, device,

@@ -67,3 +67,40 @@ def test_variants_without_history_equal_the_general_ones(make, precision, cuda):
     for options in ({"stage_tables": True}, {"no_replay": True, "stage_tables": True},
                     {"blocks_per_sm": 2}, {"blocks_per_sm": 2, "no_replay": True}):
         assert_same_run(run_tallies(spec, precision, **options), default, TOL[precision])
+
+
+def _depth(n, planes, absorb=False, absorption=False):
+    """Planes inside the sample beside the surface sensors: fluence at `planes` depths (one
+    on the interface), statistics, a field grid; `absorb`: the deepest one ends photons."""
+    spec = W.bilayer_rgd_mie(n, 6)
+    spec["sensors"] = [spec["sensors"][0]]
+    for i in range(planes):
+        spec["sensors"].append({"kind": "planar_fluence", "z": 0.125 * (i + 1), "len_x": 4.0, "len_y": 4.0,
+                                "len_t": 8.0, "dx": 0.25, "dy": 0.25, "d_t": 2.0,
+                                "absorb": absorb and i == planes - 1})
+    if planes < 5:
+        spec["sensors"] += [{"kind": "statistics", "z": 0.25, "absorb": False, "events": 64,
+                             "depth": [2.0, 16], "direction_limit": "backward"},
+                            {"kind": "planar_field", "z": 0.3, "len_x": 2.0, "len_y": 2.0, "dx": 0.25,
+                             "dy": 0.25, "absorb": False},
+                            {"kind": "farfield_fluence", "theta_max": W.PI / 2, "phi_max": 2 * W.PI,
+                             "len_t": 0.0, "d_theta": W.PI / 18, "d_phi": W.PI / 6, "d_t": 0.0}]
+    if absorption:
+        spec["absorption"] = {"radius": 3.0, "depth": 2.0, "d_r": 0.25, "d_z": 0.1}
+    return spec
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("n,planes,absorb,absorption,block", [
+    (7, 1, False, False, 0), (3001, 4, False, True, 0), (9001, 7, True, False, 64),
+    (40_000, 4, True, True, 128)])
+def test_buffered_hits_equal_hits_on_the_spot(n, planes, absorb, absorption, block, precision, cuda):
+    """Scenes with planes inside the sample buffer their hits per warp and run the photons a
+    CBS grid reads again; `no_replay` processes every hit on the spot.  The tallies, counts
+    and the Absorption grid (which the photons run again must not fill twice) are equal."""
+    spec = _depth(n, planes, absorb, absorption)
+    a = run_tallies(spec, precision, block_size=block)
+    b = run_tallies(spec, precision, no_replay=True)
+    assert a[0]["replay_launches"] == 1 and b[0]["replay_launches"] == 0
+    assert_same_run(a, b, TOL[precision])
+    assert_same_run(run_tallies(spec, precision, batch_photons=max(1, n // 3)), b, TOL[precision])
