@@ -151,21 +151,29 @@ struct Scratch {
 };
 
 // Hit queue: one entry per (photon, crossed sensor plane) whose sensors pass their
-// filters, written by the transport kernel and consumed by the tally kernel.
-// Struct-of-arrays, `cap` entries per field.
-enum QueueU32 { kQPhotonLo = 0, kQPhotonHi, kQEvents, kQMask, kQMedia, kQScene, kQU32Fields };
-enum QueueF64 { kQWeight = 0, kQOpath, kQPen, kQF64Fields };
+// filters, written by the transport kernel and consumed by the tally kernel (or a warp's
+// buffer, drain_hits).  What every hit carries is one record of whole 16-byte words (112
+// bytes in binary32, 176 in binary64), stored and loaded with 16-byte accesses: a lane
+// stores its hit with 7 instructions at one address where 28 arrays took a store and an
+// address each, run by the one or two lanes that have a hit.
+template <typename R> struct __align__(16) HitEntry {
+  double w, opath, pen;                  // weight; path length at the hit; penetration depth
+  uint32_t media, scene;                 // first species | last species << 16; sweep: the scene
+  uint32_t p_lo, p_hi, events, mask;     // photon; scattering events; sensors
+  R hit[3];                              // hit point
+  R P[9];                                // P_local at the crossing (rows m, n, s)
+  R E[4];                                // Jones vector (m.re, m.im, n.re, n.im)
+};
+static_assert(sizeof(HitEntry<float>) == 112 && sizeof(HitEntry<double>) == 176, "whole 16-byte words");
+
+// The fields only some hits have, struct-of-arrays of `cap` R each.
 enum QueueR {
-  kQHit = 0,                  // 3: hit point
-  kQP = 3,                    // 9: P_local at the crossing (rows m, n, s)
-  kQE = 12,                   // 4: Jones vector (m.re, m.im, n.re, n.im)
-  kQR1 = 16,                  // 3: r_1           -- CBS fields from here on
-  kQRn = 19,                  // 3: r_n
-  kQP1 = 22,                  // 9: frame after the first scatter
-  kQPn1 = 31,                 // 9: frame before the newest scatter
-  kQT = 40,                   // 8: interior Jones product (re, im) x 4
-  kQRFields = 48,
-  kQRBasic = 16               // fields every entry carries
+  kQR1 = 0,                   // 3: r_1           -- CBS fields
+  kQRn = 3,                   // 3: r_n
+  kQP1 = 6,                   // 9: frame after the first scatter
+  kQPn1 = 15,                 // 9: frame before the newest scatter
+  kQT = 24,                   // 8: interior Jones product (re, im) x 4
+  kQRFields = 32
 };
 
 // Likelihood-ratio ("adjoint") runs append the photon's score, one R per parameter
@@ -177,9 +185,8 @@ constexpr int kAdjMaxRadialBins = 512;
 
 struct Queue {
   unsigned long long cap;
-  uint32_t *u32;                         // [kQU32Fields][cap]
-  double *f64;                           // [kQF64Fields][cap]
-  void *r;                               // R[kQRFields][cap]
+  void *entry;                           // HitEntry<R>[cap]
+  void *r;                               // R[kQRFields + scores][cap]; null: no hit has them
 };
 
 enum ErrorFlag : unsigned int {
@@ -211,8 +218,8 @@ struct RunParams {
   lmc_record *records;                   // this launch's photons: photon_begin + i at records[i]
   Scratch *scratch;
   Queue queue;                           // used by the queued kernel pair
-  // kHitsBuffer: buffer_entries of the queue for every warp, one warp after another (the
-  // fields before kQR1 only); list_cap entries of replay_list for the photons (from
+  // kHitsBuffer: buffer_entries of the queue for every warp, one warp after another;
+  // list_cap entries of replay_list for the photons (from
   // photon_begin) whose CBS hits the rerun launch processes, with sensor_mask's sensors
   unsigned long long buffer_entries, list_cap;
   unsigned int sensor_mask;

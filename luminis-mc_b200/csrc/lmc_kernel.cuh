@@ -1976,6 +1976,35 @@ constexpr int kHitsInline = 0, kHitsQueue = 1, kHitsBuffer = 2;
 // lies on an interface can end one segment and start the next).
 __host__ __device__ constexpr unsigned hit_buffer_entries(int n_planes) { return 32 + 64 * n_planes; }
 
+template <typename R>
+__device__ __forceinline__ void store_entry(HitEntry<R> *to, const HitEntry<R> &e)
+{
+  constexpr int kN = sizeof(HitEntry<R>) / 16;
+  uint4 v[kN];
+  memcpy(v, &e, sizeof(e));
+#pragma unroll
+  for (int j = 0; j < kN; ++j)
+    reinterpret_cast<uint4 *>(to)[j] = v[j];
+}
+
+// The entry's 16 R values by 16-byte loads of their own type.
+__device__ __forceinline__ void load16(const float *from, float *v)
+{
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 t = reinterpret_cast<const float4 *>(from)[j];
+    v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
+  }
+}
+__device__ __forceinline__ void load16(const double *from, double *v)
+{
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const double2 t = reinterpret_cast<const double2 *>(from)[j];
+    v[2 * j] = t.x; v[2 * j + 1] = t.y;
+  }
+}
+
 // Append a hit to the queue (warp-aggregated slot) or (kBuffer) to the warp's buffer, whose
 // fill is
 // *fill.  Only the fields the sensors in `mask` read are written.
@@ -2006,28 +2035,24 @@ __device__ __forceinline__ void enqueue_hit(const Scene &sc, const RunParams &rp
   }
   const int tid = threadIdx.x;
   const unsigned long long C = q.cap;
-  q.u32[kQPhotonLo * C + slot] = ph.rng.p_lo;
-  q.u32[kQPhotonHi * C + slot] = ph.rng.p_hi;
-  q.u32[kQEvents * C + slot] = ph.events;
-  q.u32[kQMask * C + slot] = mask;
-  q.u32[kQMedia * C + slot] =                  // kTrack = false: the replay kernel's to write
-      kTrack ? (uint32_t)side.first_med[tid] | ((uint32_t)ph.last_med << 16) : 0u;
-  q.u32[kQScene * C + slot] = (uint32_t)ph.scene;
-  q.f64[kQWeight * C + slot] = ph.w;
-  q.f64[kQOpath * C + slot] = opath;
-  if (mask & sc.stat_mask)
-    q.f64[kQPen * C + slot] = (double)ph.pen;
-  R *r = static_cast<R *>(q.r);
-  r[(kQHit + 0) * C + slot] = hx;
-  r[(kQHit + 1) * C + slot] = hy;
-  r[(kQHit + 2) * C + slot] = hz;
+  HitEntry<R> e;
+  e.w = ph.w;
+  e.opath = opath;
+  e.pen = (double)ph.pen;
+  e.p_lo = ph.rng.p_lo;
+  e.p_hi = ph.rng.p_hi;
+  e.events = ph.events;
+  e.mask = mask;
+  // kTrack = false: the replay kernel's to write
+  e.media = kTrack ? (uint32_t)side.first_med[tid] | ((uint32_t)ph.last_med << 16) : 0u;
+  e.scene = (uint32_t)ph.scene;
+  e.hit[0] = hx; e.hit[1] = hy; e.hit[2] = hz;
 #pragma unroll
   for (int j = 0; j < 9; ++j)
-    r[(kQP + j) * C + slot] = ph.P[j];
-  r[(kQE + 0) * C + slot] = ph.Em.re;
-  r[(kQE + 1) * C + slot] = ph.Em.im;
-  r[(kQE + 2) * C + slot] = ph.En.re;
-  r[(kQE + 3) * C + slot] = ph.En.im;
+    e.P[j] = ph.P[j];
+  e.E[0] = ph.Em.re; e.E[1] = ph.Em.im; e.E[2] = ph.En.re; e.E[3] = ph.En.im;
+  store_entry(static_cast<HitEntry<R> *>(q.entry) + slot, e);
+  R *r = static_cast<R *>(q.r);
   if constexpr (kBuffer) {
     return;                              // no CBS hits here
   } else if ((mask & sc.cbs_mask) && (!kTrack || rp.cbs_replay)) {
@@ -2068,24 +2093,29 @@ __device__ __forceinline__ unsigned load_hit(const Scene &sc, const Queue &q, un
 {
   const unsigned long long C = q.cap;
   const R *r = static_cast<const R *>(q.r);
-  h.p_lo = q.u32[kQPhotonLo * C + i];
-  h.p_hi = q.u32[kQPhotonHi * C + i];
-  h.events = q.u32[kQEvents * C + i];
-  const unsigned mask = q.u32[kQMask * C + i];
-  const uint32_t media = q.u32[kQMedia * C + i];
+  const HitEntry<R> *e = static_cast<const HitEntry<R> *>(q.entry) + i;
+  const double2 wl = *reinterpret_cast<const double2 *>(&e->w);
+  const uint4 id = *reinterpret_cast<const uint4 *>(&e->p_lo);   // p_lo, p_hi, events, mask
+  const uint32_t media = e->media;
+  R v[16];
+  load16(e->hit, v);                     // hit, P, E
+  const unsigned mask = id.w;
+  h.p_lo = id.x;
+  h.p_hi = id.y;
+  h.events = id.z;
   h.first_med = media & 0xffffu;
   h.last_med = media >> 16;
-  h.w = q.f64[kQWeight * C + i];
-  h.opath = q.f64[kQOpath * C + i];
-  h.pen = (mask & sc.stat_mask) ? q.f64[kQPen * C + i] : 0.0;
-  h.hx = r[(kQHit + 0) * C + i];
-  h.hy = r[(kQHit + 1) * C + i];
-  h.hz = r[(kQHit + 2) * C + i];
+  h.w = wl.x;
+  h.opath = wl.y;
+  h.pen = (mask & sc.stat_mask) ? e->pen : 0.0;
+  h.hx = v[0];
+  h.hy = v[1];
+  h.hz = v[2];
 #pragma unroll
   for (int j = 0; j < 9; ++j)
-    h.P[j] = r[(kQP + j) * C + i];
-  h.Em = {r[(kQE + 0) * C + i], r[(kQE + 1) * C + i]};
-  h.En = {r[(kQE + 2) * C + i], r[(kQE + 3) * C + i]};
+    h.P[j] = v[3 + j];
+  h.Em = {v[12], v[13]};
+  h.En = {v[14], v[15]};
   if (kCbs && (mask & sc.cbs_mask)) {
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -2953,6 +2983,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2)
   fl.score = nullptr;
   Counters<false> cnt;
   R *r = static_cast<R *>(q.r);
+  HitEntry<R> *const entry = static_cast<HitEntry<R> *>(q.entry);
   const Scene *scp = kSweep ? g_scene : reinterpret_cast<const Scene *>(s_raw);
   unsigned long long slot = 0;
   uint32_t target = 0;
@@ -2970,10 +3001,9 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2)
         if (i < n) {
           slot = rp.replay_list[i];
           if (kSweep)
-            scp = g_scene + q.u32[kQScene * C + slot];
-          const unsigned long long index =
-              ((unsigned long long)q.u32[kQPhotonHi * C + slot] << 32) | q.u32[kQPhotonLo * C + slot];
-          target = q.u32[kQEvents * C + slot];
+            scp = g_scene + entry[slot].scene;
+          const unsigned long long index = ((unsigned long long)entry[slot].p_hi << 32) | entry[slot].p_lo;
+          target = entry[slot].events;
           init_photon<R>(*scp, rp, ph, side, index);
           busy = true;
         } else {
@@ -3001,16 +3031,16 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2)
     R dev = R(0);
 #pragma unroll
     for (int j = 0; j < 9; ++j)
-      dev = fmax(dev, fabs(ph.P[j] - r[(kQP + j) * C + slot]));
-    dev = fmax(dev, fabs(ph.Em.re - r[(kQE + 0) * C + slot]));
-    dev = fmax(dev, fabs(ph.Em.im - r[(kQE + 1) * C + slot]));
-    dev = fmax(dev, fabs(ph.En.re - r[(kQE + 2) * C + slot]));
-    dev = fmax(dev, fabs(ph.En.im - r[(kQE + 3) * C + slot]));
+      dev = fmax(dev, fabs(ph.P[j] - entry[slot].P[j]));
+    dev = fmax(dev, fabs(ph.Em.re - entry[slot].E[0]));
+    dev = fmax(dev, fabs(ph.Em.im - entry[slot].E[1]));
+    dev = fmax(dev, fabs(ph.En.re - entry[slot].E[2]));
+    dev = fmax(dev, fabs(ph.En.im - entry[slot].E[3]));
     if (ph.events != target || !(dev <= R(1e-3))) {
       atomicOr(&rp.scratch->error_flags, (unsigned)kErrReplay);
       continue;
     }
-    q.u32[kQMedia * C + slot] = (uint32_t)side.first_med[tid] | ((uint32_t)ph.last_med << 16);
+    entry[slot].media = (uint32_t)side.first_med[tid] | ((uint32_t)ph.last_med << 16);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       r[(kQR1 + j) * C + slot] = side.first[j][tid];
@@ -3072,7 +3102,7 @@ __global__ void __launch_bounds__(kBlock, (sizeof(R) == 4 && !(kAdj && kSweep)) 
   const R *r = static_cast<const R *>(q.r);
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
        i += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned scene = kSweep ? q.u32[kQScene * C + i] : 0u;
+    const unsigned scene = kSweep ? static_cast<const HitEntry<R> *>(q.entry)[i].scene : 0u;
     const Scene &sc = kSweep ? g_scene[scene] : sc0;
     HitData<R> h;
     const unsigned mask = load_hit<R>(sc, q, i, h);

@@ -1412,11 +1412,12 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
       rp.buffer_entries = dev::hit_buffer_entries(h->max_planes);
       cap = std::min<unsigned long long>(full_grid, (batch + block - 1) / block) * (block / 32) *
             rp.buffer_entries;
-      fields = dev::kQRBasic;
+      fields = 0;
       batch = std::min<unsigned long long>(batch, 1ull << 31);   // listed by 32-bit offset
       rp.list_cap = rerun ? batch : 0;   // a photon leaves through z = 0 once
     }
-    const size_t need = (size_t)cap * (dev::kQU32Fields * 4 + dev::kQF64Fields * 8 + fields * rbytes) +
+    const size_t entry = fp32 ? sizeof(dev::HitEntry<float>) : sizeof(dev::HitEntry<double>);
+    const size_t need = (size_t)cap * (entry + fields * rbytes) +
                         (size_t)rp.list_cap * sizeof(uint32_t) + 4 * 256;
     if (h->queue_bytes < need) {
       cudaFree(h->d_queue);
@@ -1431,10 +1432,8 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     unsigned char *q = static_cast<unsigned char *>(h->d_queue);
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
     rp.queue.cap = cap;
-    rp.queue.u32 = reinterpret_cast<uint32_t *>(q);
-    size_t o = align((size_t)cap * dev::kQU32Fields * 4);
-    rp.queue.f64 = reinterpret_cast<double *>(q + o);
-    o += align((size_t)cap * dev::kQF64Fields * 8);
+    rp.queue.entry = q;
+    size_t o = align((size_t)cap * entry);
     rp.queue.r = q + o;
     o += align((size_t)cap * fields * rbytes);
     rp.replay_list = rp.list_cap ? reinterpret_cast<uint32_t *>(q + o) : nullptr;
@@ -2236,8 +2235,8 @@ extern "C" lmc_status lmc_run_noalloc(const lmc_scene *s, uint64_t seed, uint64_
   per_sm = std::max(per_sm, 1);
   unsigned long long batch = n_photons;
   if (queued && n_photons > 0) {
-    const size_t entry = dev::kQU32Fields * 4 + dev::kQF64Fields * 8 +
-                         dev::kQRFields * (fp32 ? sizeof(float) : sizeof(double));
+    const size_t record = fp32 ? sizeof(dev::HitEntry<float>) : sizeof(dev::HitEntry<double>);
+    const size_t entry = record + dev::kQRFields * (fp32 ? sizeof(float) : sizeof(double));
     const unsigned long long cap = (kNoAllocBytes - kNaQueueOff - 3 * 256) / entry;
     const unsigned long long planes_n = std::max(1, n_planes);
     // cap = batch * planes + batch / 16 + 1024, as in lmc_run; a smaller batch_photons
@@ -2249,11 +2248,8 @@ extern "C" lmc_status lmc_run_noalloc(const lmc_scene *s, uint64_t seed, uint64_
       return fail(LMC_ERR_INVALID, "lmc_run_noalloc: too many sensor planes for the hit queue");
     unsigned char *q = base + kNaQueueOff;
     rp.queue.cap = cap;
-    rp.queue.u32 = reinterpret_cast<uint32_t *>(q);
-    size_t o = align((size_t)cap * dev::kQU32Fields * 4);
-    rp.queue.f64 = reinterpret_cast<double *>(q + o);
-    o += align((size_t)cap * dev::kQF64Fields * 8);
-    rp.queue.r = q + o;
+    rp.queue.entry = q;
+    rp.queue.r = q + align((size_t)cap * record);
   }
   lmc_record *const records = static_cast<lmc_record *>(opts->records);
   for (unsigned long long done = 0; done < n_photons; done += batch) {
