@@ -2718,6 +2718,131 @@ __device__ __forceinline__ void stage_amplitudes(Scene &sc, const RunParams &rp,
   }
 }
 
+// ------------------------------------------------------------ packing the launch's end
+// When no photons are left to start, a block's lanes empty one by one while its longest
+// paths (up to the event cap) go on: every warp then runs the whole event loop for one or
+// two lanes, and eight such warps per scheduler take 3-4 us per event where one alone takes
+// 1.1.  From then on the block's warps meet every kPackEvents events, and as long as the
+// live photons fit one warp fewer, the last warp's photons move to free lanes of the others.
+constexpr int kPackEvents = 16;
+
+// A photon's registers, word by word, 16 words a round, through the ring column of the lane
+// that gives it away (the ring's own words move first).
+template <bool kGive> struct Cargo {
+  uint32_t (*ring)[kBlock];
+  unsigned col;
+  int round, i;
+  __device__ __forceinline__ void word(uint32_t &v)
+  {
+    if ((i >> 4) == round) {
+      if (kGive)
+        ring[i & 15][col] = v;
+      else
+        v = ring[i & 15][col];
+    }
+    ++i;
+  }
+  __device__ __forceinline__ void operator()(uint32_t &v) { word(v); }
+  __device__ __forceinline__ void operator()(int &v)
+  {
+    uint32_t u = (uint32_t)v;
+    word(u);
+    v = (int)u;
+  }
+  __device__ __forceinline__ void operator()(float &v)
+  {
+    uint32_t u = __float_as_uint(v);
+    word(u);
+    v = __uint_as_float(u);
+  }
+  __device__ __forceinline__ void operator()(double &v)
+  {
+    uint32_t lo = (uint32_t)__double2loint(v), hi = (uint32_t)__double2hiint(v);
+    word(lo);
+    word(hi);
+    v = __hiloint2double((int)hi, (int)lo);
+  }
+};
+
+// What a photon carries between events (kPen: the penetration depth; kTrack: its newest
+// species; kSweep: its scene), the 16 R first.
+template <bool kPen, bool kTrack, bool kSweep, typename R, typename F>
+__device__ __forceinline__ int photon_words(Photon<R> &ph, F &f)
+{
+  f(ph.px); f(ph.py); f(ph.pz);
+#pragma unroll
+  for (int j = 0; j < 9; ++j)
+    f(ph.P[j]);
+  f(ph.Em.re); f(ph.Em.im); f(ph.En.re); f(ph.En.im);
+  f(ph.w); f(ph.opath);
+  f(ph.events); f(ph.layer);
+  f(ph.rng.p_lo); f(ph.rng.p_hi); f(ph.rng.draw); f(ph.rng.filled);
+  if (kPen)
+    f(ph.pen);
+  if (kTrack)
+    f(ph.last_med);
+  if (kSweep)
+    f(ph.scene);
+  return f.i;
+}
+
+// Move the photons of the block's last active warp (act - 1) to free lanes of the warps
+// before it; the caller has checked that they fit.  All threads of the block call it.
+template <typename R, bool kPen, bool kTrack, bool kSweep, bool kAdj>
+__device__ __forceinline__ void free_last_warp(const RunParams &rp, Photon<R> &ph, Side<R> &side, R *scores,
+                                               bool &alive, int act, unsigned *s_live, unsigned *s_from)
+{
+  const unsigned tid = threadIdx.x, lane = tid & 31u, lower = (1u << lane) - 1u;
+  const int warp = (int)(tid >> 5);
+  const unsigned m = __ballot_sync(kFull, alive);
+  const bool give = alive && warp == act - 1;
+  if (lane == 0)
+    s_live[warp] = (unsigned)__popc(m);
+  if (give)
+    s_from[__popc(m & lower)] = tid;
+  __syncthreads();
+  unsigned rank = (unsigned)__popc(~m & lower);
+  for (int v = 0; v < warp; ++v)
+    rank += 32u - s_live[v];
+  const bool take = !alive && warp < act - 1 && rank < s_live[act - 1];
+  const unsigned from = take ? s_from[rank] : tid;
+  if (take) {
+#pragma unroll
+    for (int j = 0; j < (int)kRing; ++j)
+      side.ring[j][tid] = side.ring[j][from];
+    if (kTrack) {
+      side.first_med[tid] = side.first_med[from];
+      if (rp.track_reverse) {            // the reverse-path history: rows of R after first_med
+        constexpr int kRows = 12 + 6 + 4 + 3 + 8;
+        static_assert(sizeof(side.first) + sizeof(side.last) + sizeof(side.ang) + sizeof(side.rn) +
+                          sizeof(side.T) == sizeof(R) * kRows * kBlock, "history rows");
+        R *row = &side.first[0][0];
+#pragma unroll 1
+        for (int j = 0; j < kRows; ++j, row += kBlock)
+          row[tid] = row[from];
+      }
+    }
+    if (kAdj)
+      for (int k = 0; k < rp.adj_K; ++k)
+        scores[k * kBlock + tid] = scores[k * kBlock + from];
+  }
+  constexpr int kWords = (16 + (kPen ? 1 : 0)) * (int)(sizeof(R) / 4) + 10 + (kTrack ? 1 : 0) + (kSweep ? 1 : 0);
+#pragma unroll
+  for (int r = 0; r < (kWords + 15) / 16; ++r) {
+    __syncthreads();                     // what the column held has been read
+    if (give) {
+      Cargo<true> out{side.ring, tid, r, 0};
+      photon_words<kPen, kTrack, kSweep>(ph, out);
+    }
+    __syncthreads();
+    if (take) {
+      Cargo<false> in{side.ring, from, r, 0};
+      photon_words<kPen, kTrack, kSweep>(ph, in);
+    }
+  }
+  alive = take || (alive && !give);
+}
+
 // kMinBlocks > 1 asks the compiler to fit that many 256-thread blocks per SM
 // (register cap 65536 / (256 kMinBlocks)); lmc_run picks the variant.
 
@@ -2799,7 +2924,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       atomicAdd(&rp.scratch->replayed, n_run);
   }
   unsigned long long *const next = listed ? &rp.scratch->replay_next : &rp.scratch->next_photon;
-  bool alive = false, done = false;
+  bool alive = false;
   __shared__ unsigned s_fill[kBlock / 32];     // kHitsBuffer: hits in each warp's buffer
   unsigned *const fill = s_fill + (threadIdx.x >> 5);
   if (kHitsTo == kHitsBuffer) {
@@ -2807,88 +2932,138 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       *fill = 0;
     __syncwarp();
   }
+  // The end of the launch is packed (free_last_warp) in the kernels where it pays: binary32
+  // with the queue, 1 M CBS photons 14.1 -> 13.0 ms, long paths (1e5 photons, cap 1e5
+  // events) 370 -> 240, gradients of a 32-medium sweep 30.2 -> 29.3, 20 M bilayer photons
+  // 165.2 -> 165.8.  Binary64 (2 M bilayer photons 44.9 -> 46.1 ms), the plain sweep (104.2
+  // -> 107.5) and the hit buffers (22.1 -> 28.4) lose more in their event loops than their
+  // ends give; the estimator's warps share their vertices.
+  constexpr bool kPack = sizeof(R) == 4 && kHitsTo == kHitsQueue && !kEst && (!kSweep || kAdj);
+  constexpr bool kPen = kTrack || kExtras;
+  __shared__ unsigned s_dry, s_live[kPack ? kBlock / 32 : 1], s_from[kPack ? 32 : 1];
+  int act = (int)(blockDim.x >> 5);      // kPack: warps that still hold photons
+  int tail = -1;                         // kPack: events since the photons ran out
+  bool done = false;                     // not kPack: no photon was left for this lane
+  if (kPack) {
+    if (threadIdx.x == 0)
+      s_dry = 0;
+    __syncthreads();
+  }
   for (;;) {
-    const unsigned need = __ballot_sync(kFull, !alive && !done);
-    if (need) {
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if ((int)lane == leader)
-        base = atomicAdd(next, (unsigned long long)__popc(need));
-      base = __shfl_sync(kFull, base, leader);
-      if (!alive && !done) {
-        const unsigned long long idx = base + __popc(need & ((1u << lane) - 1u));
-        if (idx < n_run) {
-          const unsigned long long at = rp.photon_begin + (listed ? rp.replay_list[idx] : idx);
-          int si = 0;
-          if (kSweep) {
-            si = sweep_scene(rp, at);
-            scp = g_scene + si;
+    for (;;) {
+      // lanes without a photon (kPack: none any more once the block has run dry, which every
+      // lane then asks for)
+      unsigned ask;
+      if constexpr (kPack)
+        ask = tail < 0 ? __ballot_sync(kFull, !alive || *(volatile unsigned *)&s_dry != 0u) : 0u;
+      else
+        ask = __ballot_sync(kFull, !alive && !done);
+      if (ask) {
+        const unsigned need = kPack ? __ballot_sync(kFull, !alive) : ask;
+        const int leader = __ffs(need) - 1;
+        unsigned long long base = 0;
+        if ((int)lane == leader)
+          base = atomicAdd(next, (unsigned long long)__popc(need));
+        base = __shfl_sync(kFull, base, leader & 31);
+        if (!alive && !done) {
+          const unsigned long long idx = base + __popc(need & ((1u << lane) - 1u));
+          if (idx < n_run) {
+            const unsigned long long at = rp.photon_begin + (listed ? rp.replay_list[idx] : idx);
+            int si = 0;
+            if (kSweep) {
+              si = sweep_scene(rp, at);
+              scp = g_scene + si;
+            }
+            init_photon<R, kTrack>(*scp, rp, ph, side, at);
+            ph.scene = si;
+            if (kAdj)
+              for (int k = 0; k < rp.adj_K; ++k)
+                fl[k] = R(0);
+            alive = true;
+          } else {
+            done = !kPack;
           }
-          init_photon<R, kTrack>(*scp, rp, ph, side, at);
-          ph.scene = si;
-          if (kAdj)
-            for (int k = 0; k < rp.adj_K; ++k)
-              fl[k] = R(0);
-          alive = true;
-        } else {
-          done = true;
+        }
+        if constexpr (kPack) {
+          if (base + __popc(need) > n_run || ask != need) {
+            tail = 0;
+            *(volatile unsigned *)&s_dry = 1u;
+          }
+          __syncwarp();
+        }
+      }
+      if constexpr (kPack) {
+        if (tail >= 0 && tail++ % kPackEvents == 0)
+          break;
+      } else {
+        const bool finished = __all_sync(kFull, done);
+        if constexpr (kHitsTo == kHitsBuffer) {
+          // full groups of 32 hits, all of them when the warp is done
+          __syncwarp();
+          unsigned n = *(volatile unsigned *)fill;
+          if (n >= 32u || (finished && n > 0u)) {
+            Parked<Photon<R>> parked;
+            parked.put(ph);
+            const unsigned long long first = warp_index() * rp.buffer_entries;
+            while (n >= 32u || (finished && n > 0u)) {
+              const unsigned m = n < 32u ? n : 32u;
+              n -= m;
+              drain_hits<R>(*scp, rp, first + n, m, s_hits);
+            }
+            parked.get(ph);
+            ph.rng.ring = &side.ring[0][threadIdx.x];    // shared memory, known to be so
+            if (lane == 0)
+              *fill = n;
+            __syncwarp();
+          }
+        }
+        if (finished)
+          break;
+      }
+      int fate = kAlive;
+      if constexpr (kEst) {
+        // the move, then the warp's estimate at the vertices reached (all lanes, converged),
+        // then the scatter
+        int med_idx = 0;
+        if (alive)
+          fate = event_move<R, kHitsTo, kAdj, kExtras, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, s_hits, med_idx);
+        estimate_warp<R>(*scp, rp, ph, side, med_idx, alive && fate == kAlive, s_hits, s_est);
+        if (alive && fate == kAlive)
+          fate = event_scatter<R, kAdj, kExtras, true, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, med_idx);
+      } else if (alive) {
+        fate = event_step<R, kHitsTo, kAdj, kExtras, kTrack, kTrack && !kSweep, kKeys>(*scp, rp, ph, side, fl, cnt,
+                                                                                     s_hits, fill);
+      }
+      if (alive) {
+        if (fate != kAlive) {
+          alive = false;
+          if constexpr (kCount) {
+            cnt.draws += ph.rng.draw;
+          } else {
+            add_wide(s_events, ph.events);
+            add_wide(s_draws, ph.rng.draw);
+          }
+          atomicAdd(&s_fate[fate], Fates(1));
+          if (kTrack && rp.records)
+            write_record<R>(*scp, rp, ph, side, fate);
+          if (fate == kError)
+            atomicOr(&rp.scratch->error_flags, (unsigned)kErrAborted);
+          if (!isfinite(ph.w))
+            atomicOr(&rp.scratch->error_flags, (unsigned)kErrNonFiniteWeight);
         }
       }
     }
-    const bool finished = __all_sync(kFull, done);
-    if constexpr (kHitsTo == kHitsBuffer) {
-      // full groups of 32 hits, all of them when the warp is done
-      __syncwarp();
-      unsigned n = *(volatile unsigned *)fill;
-      if (n >= 32u || (finished && n > 0u)) {
-        Parked<Photon<R>> parked;
-        parked.put(ph);
-        const unsigned long long first = warp_index() * rp.buffer_entries;
-        while (n >= 32u || (finished && n > 0u)) {
-          const unsigned m = n < 32u ? n : 32u;
-          n -= m;
-          drain_hits<R>(*scp, rp, first + n, m, s_hits);
-        }
-        parked.get(ph);
-        ph.rng.ring = &side.ring[0][threadIdx.x];    // shared memory, known to be so
-        if (lane == 0)
-          *fill = n;
-        __syncwarp();
-      }
-    }
-    if (finished)
+    if constexpr (!kPack) {
       break;
-    int fate = kAlive;
-    if constexpr (kEst) {
-      // the move, then the warp's estimate at the vertices reached (all lanes, converged),
-      // then the scatter
-      int med_idx = 0;
-      if (alive)
-        fate = event_move<R, kHitsTo, kAdj, kExtras, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, s_hits, med_idx);
-      estimate_warp<R>(*scp, rp, ph, side, med_idx, alive && fate == kAlive, s_hits, s_est);
-      if (alive && fate == kAlive)
-        fate = event_scatter<R, kAdj, kExtras, true, true, true, kKeys>(*scp, rp, ph, side, fl, cnt, med_idx);
-    } else if (alive) {
-      fate = event_step<R, kHitsTo, kAdj, kExtras, kTrack, kTrack && !kSweep, kKeys>(*scp, rp, ph, side, fl, cnt,
-                                                                                   s_hits, fill);
-    }
-    if (alive) {
-      if (fate != kAlive) {
-        alive = false;
-        if constexpr (kCount) {
-          cnt.draws += ph.rng.draw;
-        } else {
-          add_wide(s_events, ph.events);
-          add_wide(s_draws, ph.rng.draw);
-        }
-        atomicAdd(&s_fate[fate], Fates(1));
-        if (kTrack && rp.records)
-          write_record<R>(*scp, rp, ph, side, fate);
-        if (fate == kError)
-          atomicOr(&rp.scratch->error_flags, (unsigned)kErrAborted);
-        if (!isfinite(ph.w))
-          atomicOr(&rp.scratch->error_flags, (unsigned)kErrNonFiniteWeight);
-      }
+    } else {
+      const int live = __syncthreads_count(alive);
+      if (live == 0)
+        break;
+      for (; act > rp.tail_warps && live <= 32 * (act - 1); --act)
+        free_last_warp<R, kPen, kTrack, kSweep, kAdj>(rp, ph, side, reinterpret_cast<R *>(s_dyn + rp.side_off),
+                                                      alive, act, s_live, s_from);
+      if (kSweep && alive)
+        scp = g_scene + ph.scene;
     }
   }
   if constexpr (kCount) {      // warp-reduce the per-thread counters, then one atomic per warp

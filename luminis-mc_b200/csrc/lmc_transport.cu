@@ -960,6 +960,13 @@ static lmc_status sweep_adjoint_layout(const lmc_handle *h, const lmc_adjoint_op
 
 }  // extern "C"
 
+// Warps a block keeps to the end of a launch with per_sm blocks per SM: one for each of the
+// SM's four schedulers.
+static int tail_warps(int per_sm)
+{
+  return std::max(1, 4 / std::max(per_sm, 1));
+}
+
 static void set_seed(lmc::dev::RunParams &rp, uint64_t seed)
 {
   rp.key0 = (uint32_t)seed;
@@ -1399,6 +1406,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   // batches: the whole range at once inline; queue-sized batches when queued
   unsigned long long batch = n_photons;
   const unsigned long long full_grid = (unsigned long long)h->sm_count * per_sm;
+  rp.tail_warps = tail_warps(per_sm);
   if ((h->queued || buffered) && n_photons > 0) {
     batch = opts->batch_photons ? opts->batch_photons : (32ull << 20);   // ~110 B of queue per photon
     batch = std::min<unsigned long long>(batch, n_photons);
@@ -1468,6 +1476,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
         rr.rerun = 1;
         rr.track_reverse = 1;
         rr.side_off = (unsigned)dyn_replay;
+        rr.tail_warps = tail_warps(replay_grid / h->sm_count);
         rr.stage_bytes = 0;
         rr.sensor_mask = h->scene.cbs_mask;
       }
@@ -2233,6 +2242,7 @@ extern "C" lmc_status lmc_run_noalloc(const lmc_scene *s, uint64_t seed, uint64_
   if (opts->blocks_per_sm > 0)
     per_sm = std::min(per_sm, opts->blocks_per_sm);
   per_sm = std::max(per_sm, 1);
+  rp.tail_warps = tail_warps(per_sm);
   unsigned long long batch = n_photons;
   if (queued && n_photons > 0) {
     const size_t record = fp32 ? sizeof(dev::HitEntry<float>) : sizeof(dev::HitEntry<double>);

@@ -104,3 +104,45 @@ def test_buffered_hits_equal_hits_on_the_spot(n, planes, absorb, absorption, blo
     assert a[0]["replay_launches"] == 1 and b[0]["replay_launches"] == 0
     assert_same_run(a, b, TOL[precision])
     assert_same_run(run_tallies(spec, precision, batch_photons=max(1, n // 3)), b, TOL[precision])
+
+
+def _long(n):
+    spec = W.mie_long_paths(n, 8)
+    spec["max_events"] = 4000
+    return spec
+
+
+@pytest.mark.parametrize("make,n", [(W.mie_cbs_small, 1), (W.mie_cbs_small, 255), (W.mie_cbs_small, 257),
+                                    (_long, 700), (W.bilayer_rgd_mie, 5003), (_mixture_absorption, 3001)])
+@pytest.mark.parametrize("options", [{}, {"no_replay": True}, {"blocks_per_sm": 2}, {"blocks_per_sm": 1}],
+                         ids=["default", "tracked", "two_blocks", "one_block"])
+def test_packing_at_the_end_of_a_launch_changes_nothing(make, n, options, cuda):
+    """Blocks of 8 warps pack their last photons into fewer warps; blocks of one warp have
+    nothing to pack.  The same kernel computes the same photons: equal to the order of the
+    tallies' sums."""
+    spec = make(n, 8) if make in (W.mie_cbs_small, W.bilayer_rgd_mie) else make(n)
+    packed = run_tallies(spec, "fp32", block_size=256, **options)
+    assert_same_run(packed, run_tallies(spec, "fp32", block_size=32, **options), 1e-12)
+    assert_same_run(packed, run_tallies(spec, "fp32", block_size=96, **options), 1e-12)
+
+
+def test_packing_moves_records_and_scores(cuda):
+    """Every per-photon record (reverse-path history included) and the likelihood-ratio
+    scores survive the moves."""
+    from luminis_mc_b200.adjoint import AdjointTransport
+    spec = W.bilayer_rgd_mie(3000, 12)
+    recs = []
+    for block in (256, 32):
+        cfg, _, keep = W.build(lm, spec)
+        run = DeviceRun(cfg)
+        recs.append(run.run(3000, 12, precision="fp32", records=True, block_size=block)[1])
+        run.close()
+    assert recs[0].tobytes() == recs[1].tobytes()
+    # scores: two photon ranges of one launch size each against one launch
+    cfg, _, keep = W.build(lm, W.bilayer_hg(4000, 13))
+    tr = AdjointTransport(cfg, radial_sensor=1, radial_bins=20, radial_max=5.0)
+    _, whole, _ = tr.run(4000, 13)
+    parts = [tr.run(n, 13, begin=b)[1] * n for b, n in ((0, 31), (31, 1), (32, 3968))]
+    tr.close()
+    got, want = (sum(parts) / 4000).cpu().numpy(), whole.cpu().numpy()
+    np.testing.assert_allclose(got, want, rtol=0, atol=1e-12 * np.abs(want).max())
