@@ -2843,6 +2843,16 @@ __device__ __forceinline__ void free_last_warp(const RunParams &rp, Photon<R> &p
   alive = take || (alive && !give);
 }
 
+// Lanes of each warp that take an entry of a list of n when the launch has more lanes than
+// that: a warp runs each event for the lanes that are apart from one another in turn, so a
+// short list goes to as many warps as there are (1.1 us per event for a photon alone in its
+// warp, about twice that for 32 together).
+__device__ __forceinline__ unsigned spread_lanes(unsigned long long n)
+{
+  const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+  return n >= 32ull * warps ? 32u : (unsigned)((n + warps - 1) / warps);
+}
+
 // kMinBlocks > 1 asks the compiler to fit that many 256-thread blocks per SM
 // (register cap 65536 / (256 kMinBlocks)); lmc_run picks the variant.
 
@@ -2943,7 +2953,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
   __shared__ unsigned s_dry, s_live[kPack ? kBlock / 32 : 1], s_from[kPack ? 32 : 1];
   int act = (int)(blockDim.x >> 5);      // kPack: warps that still hold photons
   int tail = -1;                         // kPack: events since the photons ran out
-  bool done = false;                     // not kPack: no photon was left for this lane
+  // not kPack: no photon was left for this lane (or the list's are spread over the warps)
+  bool done = listed && lane >= spread_lanes(n_run);
   if (kPack) {
     if (threadIdx.x == 0)
       s_dry = 0;
@@ -3162,7 +3173,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2)
   const Scene *scp = kSweep ? g_scene : reinterpret_cast<const Scene *>(s_raw);
   unsigned long long slot = 0;
   uint32_t target = 0;
-  bool busy = false, done = false;
+  bool busy = false, done = lane >= spread_lanes(n);
   for (;;) {
     const unsigned need = __ballot_sync(kFull, !busy && !done);
     if (need) {

@@ -1286,9 +1286,17 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     if (adj->radial_sensor >= 0)
       dyn_tally = (size_t)(1 + rp.adj_K) * (adj->radial_bins + 1) * sizeof(double);
   }
+  // At most one warp per scheduler: the run lasts as long as its longest path, and every
+  // instruction of an event counts as latency.  The 2-block variant (no spills) with the
+  // history tracked then beats the 4-block one and a replay that walks the longest hits'
+  // paths once more: 10 k CBS photons 3.4 -> 2.2 ms (binary64 5.5 -> 3.5).  With more photons
+  // the replay costs its fixed 1.1 ms, tracking a growing share (1 M photons: 13.1 against
+  // 15.3 ms); between the two the default stays with the replay.
+  const bool short_run = n_photons <= 128ull * (unsigned)h->sm_count;
   // binary32 queued transport: a 4-block (<=64 registers, the default) and a
   // 2-block (<=128 registers) variant; blocks_per_sm == 1 or 2 selects the latter
-  const bool wide = fp32 && h->queued && !adj && (opts->blocks_per_sm == 0 || opts->blocks_per_sm >= 3);
+  const bool wide = fp32 && h->queued && !adj &&
+                    (opts->blocks_per_sm == 0 ? !short_run : opts->blocks_per_sm >= 3);
   bool extras = false;
   for (int k = 0; k < h->n_scenes; ++k)
     extras = extras || scene_extras(sw ? h->scenes[k] : h->scene);
@@ -1308,7 +1316,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   bool any_cbs = false;
   for (int k = 0; k < h->n_scenes; ++k)
     any_cbs = any_cbs || (sw ? h->scenes[k] : h->scene).cbs_mask != 0;
-  const bool replay = h->queued && !est && !opts->records && !opts->no_replay &&
+  const bool replay = h->queued && !est && !opts->records && !opts->no_replay && !short_run &&
                       opts->track_reverse_paths && any_cbs;
   rp.cbs_replay = replay ? 1 : 0;
   // Planes inside the sample: hits go through the warps' buffers, and the photons whose CBS

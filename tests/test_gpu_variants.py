@@ -57,10 +57,12 @@ def assert_same_run(a, b, tol):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("n", [301, 19_001], ids=["short_run", "long_run"])
 @pytest.mark.parametrize("make", [_fluence_only, _statistics, _mixture_absorption],
                          ids=["fluence_only", "statistics", "mixture_absorption"])
-def test_variants_without_history_equal_the_general_ones(make, precision, cuda):
-    spec = make(12_001)
+def test_variants_without_history_equal_the_general_ones(make, n, precision, cuda):
+    """(runs of at most 128 photons per SM track the history instead of replaying)"""
+    spec = make(n)
     default = run_tallies(spec, precision)
     assert default[0]["events"] > 0
     # (two blocks per SM: the kernels that count events per thread, not per block)
