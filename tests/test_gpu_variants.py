@@ -148,3 +148,12 @@ def test_packing_moves_records_and_scores(cuda):
     tr.close()
     got, want = (sum(parts) / 4000).cpu().numpy(), whole.cpu().numpy()
     np.testing.assert_allclose(got, want, rtol=0, atol=1e-12 * np.abs(want).max())
+
+
+@pytest.mark.parametrize("n_div", [1, 2, 127, 1022, 1023, 1024, 2500])
+def test_batched_cdf_at_chunk_edges(n_div, cuda):
+    """The batched tables' CDF sums run in chunks of 1024 nodes: bit for bit the host's."""
+    species = [(W.LAMBDA, r, W.N_SPHERE, W.N_WATER) for r in (0.05e-3, 0.4e-3, 2.0e-3)]
+    for (ph, _), q in zip(lm.mie_species(species, n_div, 0.2, 2.9), species):
+        ref = lm.MiePhaseFunction(*q, n_div, 0.2, 2.9)
+        np.testing.assert_array_equal(ph._table()[1], ref._table()[1])
