@@ -224,6 +224,7 @@ struct RunParams {
   unsigned long long buffer_entries, list_cap;
   unsigned int sensor_mask;
   int rerun;
+  unsigned int est_lanes;                // estimator: lanes of a warp that take photons
   int tail_warps;                        // warps a block keeps when the launch runs out of photons
   unsigned int cbs_mask;                 // sensors whose hits need the CBS fields
   unsigned int pad;

@@ -2953,8 +2953,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
   __shared__ unsigned s_dry, s_live[kPack ? kBlock / 32 : 1], s_from[kPack ? 32 : 1];
   int act = (int)(blockDim.x >> 5);      // kPack: warps that still hold photons
   int tail = -1;                         // kPack: events since the photons ran out
-  // not kPack: no photon was left for this lane (or the list's are spread over the warps)
-  bool done = listed && lane >= spread_lanes(n_run);
+  // not kPack: no photon was left for this lane (or it takes none: spread_lanes, est_lanes)
+  bool done = (listed && lane >= spread_lanes(n_run)) || (kEst && lane >= rp.est_lanes);
   if (kPack) {
     if (threadIdx.x == 0)
       s_dry = 0;

@@ -1415,6 +1415,14 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   unsigned long long batch = n_photons;
   const unsigned long long full_grid = (unsigned long long)h->sm_count * per_sm;
   rp.tail_warps = tail_warps(per_sm);
+  // The estimator's warp takes its lanes' vertices one after another, so a warp's event costs
+  // what its photons' estimates cost together: with fewer photons than lanes, every warp of
+  // the GPU gets a few instead of the first warps 32 each.  100 bins, 3 k photons: 80 -> 26
+  // ms, 20 k: 89 -> 54; binary64, 10 k: 182 -> 92.  (Fewer lanes than that for more photons
+  // lose: the transport's own part of an event is per warp.)
+  const unsigned long long warps = full_grid * (block / 32);
+  rp.est_lanes = (unsigned)std::min(32ull, std::max(1ull, (n_photons + warps - 1) / warps));
+  const unsigned long long block_photons = (unsigned long long)(block / 32) * (est ? rp.est_lanes : 32u);
   if ((h->queued || buffered) && n_photons > 0) {
     batch = opts->batch_photons ? opts->batch_photons : (32ull << 20);   // ~110 B of queue per photon
     batch = std::min<unsigned long long>(batch, n_photons);
@@ -1426,7 +1434,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
       rp.list_cap = replay ? cap : 0;
     } else {                             // one buffer per warp of the launch
       rp.buffer_entries = dev::hit_buffer_entries(h->max_planes);
-      cap = std::min<unsigned long long>(full_grid, (batch + block - 1) / block) * (block / 32) *
+      cap = std::min<unsigned long long>(full_grid, (batch + block_photons - 1) / block_photons) * (block / 32) *
             rp.buffer_entries;
       fields = 0;
       batch = std::min<unsigned long long>(batch, 1ull << 31);   // listed by 32-bit offset
@@ -1472,7 +1480,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     // reset the work counters (transport, replay) and the queue fills of this batch
     LMC_CUDA(cudaMemsetAsync(h->d_scratch, 0, 4 * sizeof(unsigned long long), stream));
     const int grid = (int)std::max<unsigned long long>(
-        1ull, std::min<unsigned long long>(full_grid, (nb + block - 1) / block));
+        1ull, std::min<unsigned long long>(full_grid, (nb + block_photons - 1) / block_photons));
     const size_t pair = 2 * (size_t)(done / batch);
     if (stats)
       LMC_CUDA(cudaEventRecord(h->kev[pair], stream));

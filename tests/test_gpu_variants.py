@@ -157,3 +157,14 @@ def test_batched_cdf_at_chunk_edges(n_div, cuda):
     for (ph, _), q in zip(lm.mie_species(species, n_div, 0.2, 2.9), species):
         ref = lm.MiePhaseFunction(*q, n_div, 0.2, 2.9)
         np.testing.assert_array_equal(ph._table()[1], ref._table()[1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("n,bins", [(1, 40), (37, 100), (2500, 33)])
+def test_spread_estimator_runs_equal_dense_ones(n, bins, precision, cuda):
+    """Estimator runs with fewer photons than lanes spread them over all warps; one block per
+    SM of one warp holds them densely.  Same estimates, other order of the sums."""
+    spec = W.mie_cbs_small(n, 21)
+    spec["sensors"] = [dict(spec["sensors"][0], estimator=True, d_theta=0.1 / bins)]
+    spread = run_tallies(spec, precision)
+    assert_same_run(spread, run_tallies(spec, precision, block_size=32, blocks_per_sm=1), 1e-12)
