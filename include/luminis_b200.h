@@ -224,7 +224,7 @@ typedef struct lmc_run_opts {
   int blocks_per_sm;            /* 0: as many as fit                                   */
   void *records;                /* optional device array of n_photons lmc_record       */
   void *stream;                 /* cudaStream_t to launch on; NULL: the handle's own   */
-  uint64_t batch_photons;       /* photons per transport batch (hit-queue mode); 0: 32 Mi */
+  uint64_t batch_photons;       /* photons per transport batch; 0: 32 Mi                */
   int stream_format;            /* 0: u24 for FP32, u53 for FP64; 1: u24 for both (an FP64
                                    run on the FP32 run's numbers: precision alone)      */
   int host_tallies_zero;        /* lmc_run_host only: the caller's host tallies are all zero,
@@ -236,8 +236,10 @@ typedef struct lmc_run_opts {
                                    that keeps the blocks per SM; 0 reads them through L1  */
   int no_replay;                /* 1: the transport keeps every photon's reverse-path history
                                    instead of replaying the photons a FarFieldCBS grid reads
-                                   (replay is used by queued runs without records or
-                                   estimator sensors, likelihood-ratio runs included)     */
+                                   (replay is used by queued runs of more than 128 photons
+                                   per SM without records or estimator sensors, likelihood-
+                                   ratio runs included).  With planes inside the sample:
+                                   every hit processed on the spot, none buffered          */
   int tally_mode;               /* lmc_tally_mode of the hit-queue tally kernel (queued
                                    runs; inline runs add with global atomics)             */
 } lmc_run_opts;
@@ -265,7 +267,7 @@ typedef struct lmc_stats {
   float kernel_ms;                  /* whole run on the device (all launches), CUDA events */
   float transport_ms;               /* sum of the transport kernel launches alone       */
   uint32_t transport_launches;      /* transport kernel launches (queue batches)        */
-  uint32_t replay_launches;         /* CBS replay kernel launches (0: no replay)        */
+  uint32_t replay_launches;         /* CBS replay (or rerun) launches (0: no replay)    */
   uint64_t replayed;                /* photons whose reverse path the replay rebuilt    */
 } lmc_stats;
 

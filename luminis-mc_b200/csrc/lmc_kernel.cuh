@@ -11,10 +11,9 @@
 // reference's do not depend on n_threads.
 //
 // State layout: what every event reads lives in registers (position, frame,
-// Jones vector, weight, the running interior Jones product, the previous frame
-// and position); what only a CBS detection reads -- the first-scatter frame and
-// position and the newest event's raw Jones factors -- lives in shared memory,
-// one slot per thread.  The emission time is recomputed from the counter-based
+// Jones vector, weight); the photon's random words, and in launches that keep it
+// the reverse-path history a CBS detection reads, live in shared memory, one
+// column per thread.  The emission time is recomputed from the counter-based
 // stream when a detector needs it instead of being carried.
 //
 // Precision: `R` is the transport type (float or double).  The weight, the
@@ -2005,9 +2004,8 @@ __device__ __forceinline__ void load16(const double *from, double *v)
   }
 }
 
-// Append a hit to the queue (warp-aggregated slot) or (kBuffer) to the warp's buffer, whose
-// fill is
-// *fill.  Only the fields the sensors in `mask` read are written.
+// Append a hit to the queue (warp-aggregated slot) or (kBuffer) to the warp's buffer, which
+// holds *fill hits.  The CBS fields and the scores are written where they are needed only.
 template <typename R, bool kAdj, bool kTrack, bool kBuffer>
 __device__ __forceinline__ void enqueue_hit(const Scene &sc, const RunParams &rp, const Photon<R> &ph,
                                             const Side<R> &side, const Flight<R> &fl, R t,
@@ -3012,6 +3010,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
           // full groups of 32 hits, all of them when the warp is done
           __syncwarp();
           unsigned n = *(volatile unsigned *)fill;
+          if (n > rp.buffer_entries)       // reported as an overflow (enqueue_hit)
+            n = (unsigned)rp.buffer_entries;
           if (n >= 32u || (finished && n > 0u)) {
             Parked<Photon<R>> parked;
             parked.put(ph);

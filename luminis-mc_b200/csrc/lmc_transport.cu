@@ -1443,11 +1443,26 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     const size_t entry = fp32 ? sizeof(dev::HitEntry<float>) : sizeof(dev::HitEntry<double>);
     const size_t need = (size_t)cap * (entry + fields * rbytes) +
                         (size_t)rp.list_cap * sizeof(uint32_t) + 4 * 256;
+    // The buffers speed a run up that also goes without them: on the spot where they cannot
+    // be had (no memory, or a stream capture that may not allocate)
+    auto on_the_spot = [&] {
+      lmc_run_opts o = *opts;
+      o.no_replay = 1;
+      return run_impl(h, seed, photon_begin, n_photons, &o, adj, d_adj, d_tallies, stats);
+    };
     if (h->queue_bytes < need) {
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      if (buffered && cudaStreamIsCapturing(stream, &capture) == cudaSuccess &&
+          capture != cudaStreamCaptureStatusNone)
+        return on_the_spot();
       cudaFree(h->d_queue);
       h->d_queue = nullptr;
       h->queue_bytes = 0;
       const cudaError_t e = cudaMalloc(&h->d_queue, need);
+      if (e != cudaSuccess && buffered) {
+        cudaGetLastError();
+        return on_the_spot();
+      }
       if (e != cudaSuccess)
         return fail(e == cudaErrorMemoryAllocation ? LMC_ERR_NOMEM : LMC_ERR_CUDA,
                     std::string("hit queue allocation: ") + cudaGetErrorString(e));

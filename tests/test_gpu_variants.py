@@ -168,3 +168,25 @@ def test_spread_estimator_runs_equal_dense_ones(n, bins, precision, cuda):
     spec["sensors"] = [dict(spec["sensors"][0], estimator=True, d_theta=0.1 / bins)]
     spread = run_tallies(spec, precision)
     assert_same_run(spread, run_tallies(spec, precision, block_size=32, blocks_per_sm=1), 1e-12)
+
+
+def test_first_run_of_a_scene_with_inner_planes_can_be_captured(cuda):
+    """Under stream capture nothing may be allocated: a scene with inner planes whose buffers
+    do not exist yet then processes its hits on the spot."""
+    import torch
+    spec = _depth(2000, 2)
+    stats, want = run_tallies(spec, "fp32", no_replay=True)
+    cfg, _, keep = W.build(lm, spec)
+    run = DeviceRun(cfg)
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        run.transport.run_device(run.tallies.data_ptr(), 2000, spec["seed"], want_stats=False,
+                                 stream=stream.cuda_stream)
+    for _ in range(2):
+        run.zero()
+        graph.replay()
+        for x, y in zip(run.host_tallies(), want):
+            np.testing.assert_allclose(x, y, rtol=0, atol=1e-12 * max(np.abs(y).max(), 1e-300))
+    del graph
+    run.close()
