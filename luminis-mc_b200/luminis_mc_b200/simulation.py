@@ -367,8 +367,14 @@ _cache: list = []                    # [digest, Transport] of the last scene
 
 
 def _scene_digest(desc) -> bytes:
+    # by value: the table pointers are left out (their contents follow), or the same scene
+    # built again would miss the kept one and pay for its tables, queue and buffers again
+    # (10 k CBS photons 3.9 ms a call against 2.4, binary64 bilayer 2 M 50.5 against 46.6)
     sc, keep, _ = desc
-    h = hashlib.blake2b(bytes(sc), digest_size=32)
+    image = N.SceneDesc.from_buffer_copy(sc)
+    for m in image.media[:image.n_media]:
+        m.theta_values = m.theta_cdf = m.amp_s1 = m.amp_s2 = N.dptr()
+    h = hashlib.blake2b(bytes(image), digest_size=32)
     for a in keep:
         if isinstance(a, np.ndarray):
             h.update(np.ascontiguousarray(a).view(np.uint8).tobytes())
