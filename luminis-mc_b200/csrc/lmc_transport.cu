@@ -1323,8 +1323,13 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   // hits a grid reads are run again with their history.  Records keep a photon's last hit,
   // which needs its hits in order, and a CBS plane above z = 0 could list a photon twice:
   // those runs (and no_replay) process every hit on the spot.
+  // So do short runs with a CBS sensor, which the rerun would make walk their longest paths
+  // twice: buffered against on the spot, binary32 150 k photons 9.3 / 7.1 ms, 300 k 10.6 /
+  // 14.5; binary64 40 k 9.2 / 7.9, 80 k 10.3 / 10.5.  Without one the buffers are level or
+  // faster from the smallest runs on (5 k 3.4 / 3.4, 300 k 7.6 / 14.0).
+  const unsigned long long spot_photons = any_cbs ? (fp32 ? 1280ull : 512ull) * (unsigned)h->sm_count : 0;
   const bool buffered = !h->queued && !opts->records && !opts->no_replay && !h->deep_cbs &&
-                        h->tally_doubles > 0;
+                        h->tally_doubles > 0 && n_photons > spot_photons;
   const bool rerun = buffered && any_cbs;
   rp.sensor_mask = ~0u;
   const bool track = (!h->queued && !buffered) || est || opts->records || opts->stage_tables ||
