@@ -3007,9 +3007,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       } else {
         const bool finished = __all_sync(kFull, done);
         if constexpr (kHitsTo == kHitsBuffer) {
-          // full groups of 32 hits, all of them when the warp is done
+          // full groups of 32 hits, all of them when the warp is done.  One lane reads the
+          // fill for all: the lanes agree on n (drain_hits needs the whole warp), and none
+          // adds the hits of its next event before the read.
           __syncwarp();
-          unsigned n = *(volatile unsigned *)fill;
+          unsigned n = lane == 0 ? *(volatile unsigned *)fill : 0u;
+          n = __shfl_sync(kFull, n, 0);
           if (n > rp.buffer_entries)       // reported as an overflow (enqueue_hit)
             n = (unsigned)rp.buffer_entries;
           if (n >= 32u || (finished && n > 0u)) {
