@@ -297,7 +297,11 @@ LMC_API lmc_status lmc_tally_layout(const lmc_handle *h, int sensor, size_t *off
  * lmc_tally_layout(-1)).  Replaces the worker loop and merge of
  * run_simulation_parallel (src/simulation.cpp:157-243) and run_photon
  * (src/simulation.cpp:255-617).  Asynchronous on the handle's stream except for
- * the statistics read-back when `stats` is non-NULL. */
+ * the statistics read-back when `stats` is non-NULL.
+ * With `stats` NULL it can be captured in a CUDA graph after one uncaptured call of the
+ * same size, which allocates the hit queue; a scene with sensor planes inside the sample
+ * also before one (its hits are then processed on the spot).  The graph stays valid until
+ * lmc_destroy: a queue that a capture recorded is kept when a larger call outgrows it. */
 LMC_API lmc_status lmc_run(lmc_handle *h, uint64_t seed, uint64_t photon_begin, uint64_t n_photons,
                    const lmc_run_opts *opts, double *d_tallies, lmc_stats *stats);
 

@@ -86,8 +86,10 @@ struct lmc_handle {
   std::vector<cudaEvent_t> kev;          // per transport launch: start, end
   double *d_host_tally = nullptr;        // staging for lmc_run_host
   size_t host_tally_cap = 0;
-  void *d_queue = nullptr;               // hit queue (queued mode), grown on demand
+  void *d_queue = nullptr;               // hit queue or warp buffers, grown on demand
   size_t queue_bytes = 0;
+  bool queue_captured = false;           // a stream capture recorded d_queue's address
+  std::vector<void *> outgrown;          // queues that were, kept for their graphs
   unsigned cbs_mask = 0;                 // sensors that need the CBS fields of a hit
   bool queued = false;                   // every sensor plane at z <= 0: queued kernel pair
   int max_planes = 0;                    // most sensor planes of any scene
@@ -834,6 +836,8 @@ void lmc_destroy(lmc_handle *h)
   cudaFree(h->d_scratch);
   cudaFree(h->d_host_tally);
   cudaFree(h->d_queue);
+  for (void *q : h->outgrown)
+    cudaFree(q);
   cudaFree(h->d_prefix);
   cudaFree(h->d_sweep_hits);
   cudaFree(h->d_adj_scenes);
@@ -1455,12 +1459,17 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
       o.no_replay = 1;
       return run_impl(h, seed, photon_begin, n_photons, &o, adj, d_adj, d_tallies, stats);
     };
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    LMC_CUDA(cudaStreamIsCapturing(stream, &capture));
+    const bool capturing = capture != cudaStreamCaptureStatusNone;
     if (h->queue_bytes < need) {
-      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-      if (buffered && cudaStreamIsCapturing(stream, &capture) == cudaSuccess &&
-          capture != cudaStreamCaptureStatusNone)
+      if (buffered && capturing)
         return on_the_spot();
-      cudaFree(h->d_queue);
+      if (h->queue_captured)             // a graph may still write to it
+        h->outgrown.push_back(h->d_queue);
+      else
+        cudaFree(h->d_queue);
+      h->queue_captured = false;
       h->d_queue = nullptr;
       h->queue_bytes = 0;
       const cudaError_t e = cudaMalloc(&h->d_queue, need);
@@ -1473,6 +1482,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
                     std::string("hit queue allocation: ") + cudaGetErrorString(e));
       h->queue_bytes = need;
     }
+    h->queue_captured |= capturing;
     unsigned char *q = static_cast<unsigned char *>(h->d_queue);
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
     rp.queue.cap = cap;

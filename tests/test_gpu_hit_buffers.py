@@ -1,8 +1,11 @@
 """Scenes with sensor planes inside the sample: hits buffered per warp, and the photons a
 FarFieldCBS grid reads run again, against every hit processed on the spot (`no_replay`)."""
+import numpy as np
 import pytest
 
+import luminis_mc_b200 as lm
 from luminis_mc_b200 import workloads as W
+from luminis_mc_b200.device import DeviceRun
 from tests.test_gpu_variants import TOL, assert_same_run, run_tallies
 
 pytestmark = pytest.mark.gpu
@@ -33,3 +36,39 @@ def test_buffers_filled_many_times_over_lose_no_hit(n, planes, block, precision,
     assert sum(want[0]["hits"]) > n
     for _ in range(3):
         assert_same_run(run_tallies(spec, precision, block_size=block), want, TOL[precision])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("make,n", [(lambda n: _planes(n, 3, cone=True), 200_003), (lambda n: _planes(n, 2), 2000),
+                                    (lambda n: W.mie_cbs_small(n, 31), 20_000)],
+                         ids=["planes_and_cone", "planes", "queue"])
+def test_a_captured_run_survives_larger_runs(make, n, precision, cuda):
+    """The queue and the warps' buffers grow with the run.  A graph captured after a run of
+    its size holds their address: it still gives the same run when larger runs on the handle
+    have outgrown them, and so does one captured after that."""
+    import torch
+    spec = make(n)
+    stats, want = run_tallies(spec, precision)
+    cfg, _, keep = W.build(lm, spec)
+    run = DeviceRun(cfg)
+    stream = torch.cuda.Stream()
+
+    def capture():
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            run.transport.run_device(run.tallies.data_ptr(), n, spec["seed"], want_stats=False,
+                                     precision=precision, stream=stream.cuda_stream)
+        return graph
+
+    run.run(n, 1, precision=precision)
+    graphs = [capture()]
+    for larger in (2 * n, 5 * n):
+        assert run.run(larger, 2, precision=precision)[0]["error_flags"] == 0
+        graphs.append(capture())
+    for graph in graphs:
+        run.zero()
+        graph.replay()
+        for x, y in zip(run.host_tallies(), want):
+            np.testing.assert_allclose(x, y, rtol=0, atol=1e-12 * max(np.abs(y).max(), 1e-300))
+    del graph, graphs
+    run.close()
