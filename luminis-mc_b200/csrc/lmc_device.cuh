@@ -189,11 +189,19 @@ struct Queue {
   void *r;                               // R[kQRFields + scores][cap]; null: no hit has them
 };
 
+// kHitsBuffer: a photon whose exit a FarFieldCBS grid sees, listed to be run again, with
+// what the rerun compares its walk with.
+struct __align__(16) RerunEntry {
+  uint32_t photon;                       // from RunParams::photon_begin
+  uint32_t events;                       // scattering events at the exit
+  float ux, uy;                          // exit direction
+};
+
 enum ErrorFlag : unsigned int {
   kErrNonFiniteWeight = 1u << 0,   // a photon ended with a NaN/inf weight
   kErrAborted = 1u << 1,           // a photon was dropped: non-finite state (see kError)
   kErrQueueOverflow = 1u << 2,     // more hits than the queue holds (tallies incomplete)
-  kErrReplay = 1u << 3,            // a replayed history did not reach its recorded hit
+  kErrReplay = 1u << 3,            // a replayed history did not reach its recorded hit or exit
   kErrStaging = 1u << 4,           // a table copy into shared memory did not complete in time
 };
 
@@ -219,8 +227,8 @@ struct RunParams {
   Scratch *scratch;
   Queue queue;                           // used by the queued kernel pair
   // kHitsBuffer: buffer_entries of the queue for every warp, one warp after another;
-  // list_cap entries of replay_list for the photons (from
-  // photon_begin) whose CBS hits the rerun launch processes, with sensor_mask's sensors
+  // list_cap RerunEntry at replay_list for the photons whose CBS hits the rerun launch
+  // processes, with sensor_mask's sensors
   unsigned long long buffer_entries, list_cap;
   unsigned int sensor_mask;
   int rerun;
@@ -255,7 +263,7 @@ struct RunParams {
   // and the replay kernel rebuilds those photons' histories from their streams
   int cbs_replay;
   int cbs_phase_f32;                     // the CBS geometric phase in binary32 (precision study)
-  uint32_t *replay_list;
+  void *replay_list;                     // uint32_t[list_cap] (kHitsBuffer: RerunEntry)
   // amplitude tables staged per block: every medium's amp_f, one after another, copied
   // by cp.async.bulk into dynamic shared memory at byte stage_off (0 bytes: not staged)
   unsigned int stage_bytes, stage_off;

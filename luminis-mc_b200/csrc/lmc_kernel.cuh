@@ -2058,7 +2058,7 @@ __device__ __forceinline__ void enqueue_hit(const Scene &sc, const RunParams &rp
     if (needs_reverse<R>(sc, mask, ph)) {
       const unsigned long long k = atomicAdd(&rp.scratch->replay_count, 1ull);
       if (k < C)
-        rp.replay_list[k] = (uint32_t)slot;
+        static_cast<uint32_t *>(rp.replay_list)[k] = (uint32_t)slot;
     }
   } else if (kTrack && (mask & sc.cbs_mask)) {
 #pragma unroll
@@ -2216,7 +2216,10 @@ __device__ __forceinline__ bool record_hit(const Scene &sc, const RunParams &rp,
         if ((mask & sc.cbs_mask) && sees_cbs_grid<R>(sc, mask, ph)) {
           const unsigned long long k = atomicAdd(&rp.scratch->replay_count, 1ull);
           if (k < rp.list_cap)
-            rp.replay_list[k] = (uint32_t)(ph.index() - rp.photon_begin);
+            static_cast<RerunEntry *>(rp.replay_list)[k] = {(uint32_t)(ph.index() - rp.photon_begin), ph.events,
+                                                            (float)ph.P[6], (float)ph.P[7]};
+          else
+            atomicOr(&rp.scratch->error_flags, (unsigned)kErrQueueOverflow);
         }
         mask &= ~sc.cbs_mask;
         if (mask)
@@ -2932,6 +2935,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       atomicAdd(&rp.scratch->replayed, n_run);
   }
   unsigned long long *const next = listed ? &rp.scratch->replay_next : &rp.scratch->next_photon;
+  const RerunEntry *const list = static_cast<const RerunEntry *>(rp.replay_list);
+  uint32_t entry = 0;                    // listed: this lane's photon in it
   bool alive = false;
   __shared__ unsigned s_fill[kBlock / 32];     // kHitsBuffer: hits in each warp's buffer
   unsigned *const fill = s_fill + (threadIdx.x >> 5);
@@ -2977,7 +2982,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
         if (!alive && !done) {
           const unsigned long long idx = base + __popc(need & ((1u << lane) - 1u));
           if (idx < n_run) {
-            const unsigned long long at = rp.photon_begin + (listed ? rp.replay_list[idx] : idx);
+            unsigned long long at = rp.photon_begin + idx;
+            if constexpr (kHitsTo == kHitsInline)
+              if (listed) {
+                entry = (uint32_t)idx;
+                at = rp.photon_begin + list[idx].photon;
+              }
             int si = 0;
             if (kSweep) {
               si = sweep_scene(rp, at);
@@ -3064,6 +3074,13 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
             atomicOr(&rp.scratch->error_flags, (unsigned)kErrAborted);
           if (!isfinite(ph.w))
             atomicOr(&rp.scratch->error_flags, (unsigned)kErrNonFiniteWeight);
+          if constexpr (kHitsTo == kHitsInline)
+            if (listed) {                // the same walk as the first: event count and exit
+              const RerunEntry w = list[entry];
+              if (fate != kDetected || ph.events != w.events || !(fabs(ph.P[6] - R(w.ux)) <= R(1e-3)) ||
+                  !(fabs(ph.P[7] - R(w.uy)) <= R(1e-3)))
+                atomicOr(&rp.scratch->error_flags, (unsigned)kErrReplay);
+            }
         }
       }
     }
@@ -3188,7 +3205,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2)
       if (!busy && !done) {
         const unsigned long long i = base + __popc(need & ((1u << lane) - 1u));
         if (i < n) {
-          slot = rp.replay_list[i];
+          slot = static_cast<const uint32_t *>(rp.replay_list)[i];
           if (kSweep)
             scp = g_scene + entry[slot].scene;
           const unsigned long long index = ((unsigned long long)entry[slot].p_hi << 32) | entry[slot].p_lo;

@@ -1451,7 +1451,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     }
     const size_t entry = fp32 ? sizeof(dev::HitEntry<float>) : sizeof(dev::HitEntry<double>);
     const size_t need = (size_t)cap * (entry + fields * rbytes) +
-                        (size_t)rp.list_cap * sizeof(uint32_t) + 4 * 256;
+                        (size_t)rp.list_cap * (rerun ? sizeof(dev::RerunEntry) : sizeof(uint32_t)) + 4 * 256;
     // The buffers speed a run up that also goes without them: on the spot where they cannot
     // be had (no memory, or a stream capture that may not allocate)
     auto on_the_spot = [&] {
@@ -1490,7 +1490,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     size_t o = align((size_t)cap * entry);
     rp.queue.r = q + o;
     o += align((size_t)cap * fields * rbytes);
-    rp.replay_list = rp.list_cap ? reinterpret_cast<uint32_t *>(q + o) : nullptr;
+    rp.replay_list = rp.list_cap ? q + o : nullptr;
   }
   if (stats && n_photons > 0) {           // one event pair per transport launch
     const size_t need_ev = 2 * (size_t)((n_photons + batch - 1) / batch);

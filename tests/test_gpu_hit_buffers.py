@@ -72,3 +72,13 @@ def test_a_captured_run_survives_larger_runs(make, n, precision, cuda):
             np.testing.assert_allclose(x, y, rtol=0, atol=1e-12 * max(np.abs(y).max(), 1e-300))
     del graph, graphs
     run.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("batch", [0, 60_000])
+def test_the_rerun_takes_every_photon_the_cone_sees(batch, precision, cuda):
+    """The cone's filter is its grid, so every photon it detects is listed, once, and run
+    again; a rerun that left the listed walk would raise an error flag."""
+    stats, _ = run_tallies(_planes(200_003, 2, cone=True), precision, batch_photons=batch)
+    assert stats["replay_launches"] == (4 if batch else 1) and stats["error_flags"] == 0
+    assert stats["replayed"] == stats["detected"] == stats["hits"][0] > 100
