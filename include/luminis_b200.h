@@ -233,7 +233,9 @@ typedef struct lmc_run_opts {
                                    0 in binary64 (default), 1 in binary32 (precision study) */
   int stage_tables;             /* binary32 transport: copy every medium's amplitude table
                                    into each block's shared memory (1-D bulk copies) when
-                                   that keeps the blocks per SM; 0 reads them through L1  */
+                                   that keeps the blocks per SM; 0 reads them through L1,
+                                   as do runs that buffer the hits of planes inside the
+                                   sample                                                */
   int no_replay;                /* 1: the transport keeps every photon's reverse-path history
                                    instead of replaying the photons a FarFieldCBS grid reads
                                    (replay is used by queued runs of more than 128 photons

@@ -1016,10 +1016,8 @@ static KernelFn pick_transport_e(bool fp32, bool queued, bool wide, bool adj, bo
   if (!queued && !buffered)
     return fp32 ? transport_kernel<float, kHitsInline, 1, false, false, false, E>
                 : transport_kernel<double, kHitsInline, 1, false, false, false, E>;
+  // (without the history, which their runs never keep)
   // binary32 at 4 blocks per SM: 22.9 ms for 1 M photons with 5 planes, 25.2 at 3, 28.8 at 2
-  if (!queued && track)
-    return fp32 ? transport_kernel<float, kHitsBuffer, 4, false, false, false, E>
-                : transport_kernel<double, kHitsBuffer, 2, false, false, false, E>;
   if (!queued)
     return fp32 ? transport_kernel<float, kHitsBuffer, 4, false, false, false, E, false>
                 : transport_kernel<double, kHitsBuffer, 2, false, false, false, E, false>;
@@ -1336,7 +1334,12 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
                         h->tally_doubles > 0 && n_photons > spot_photons;
   const bool rerun = buffered && any_cbs;
   rp.sensor_mask = ~0u;
-  const bool track = (!h->queued && !buffered) || est || opts->records || opts->stage_tables ||
+  // Staged tables are a matter of the kernels with the history: with the buffers' shared
+  // memory and registers they lost (4 M bilayer photons with three planes and the cone 65.2
+  // against 64.0 ms, 4 M with one plane 57.1 / 53.0; binary64, which stages nothing, 86.0 /
+  // 67.6 for the history's code alone), so buffered runs read them through L1.
+  const bool staged = opts->stage_tables && !buffered;
+  const bool track = (!h->queued && !buffered) || est || opts->records || staged ||
                      (any_cbs && !replay && !rerun);
   // StatisticsSensors read the penetration depth, which the queued variants without history
   // carry beside the extras only
@@ -1388,7 +1391,7 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
     rp.est_smem_doubles = (int)(rp.est_per_warp ? (block / 32) * est_block_doubles : est_block_doubles);
     dyn_transport += (size_t)rp.est_smem_doubles * sizeof(double);
   }
-  if (opts->stage_tables && fp32 && !sw) {
+  if (staged && fp32 && !sw) {
     // every medium's binary32 amplitude table in the block's shared memory, after the
     // other dynamic arrays -- as long as that keeps the blocks per SM
     size_t bytes = 0;
@@ -1521,9 +1524,6 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
       if (rerun) {
         rr.rerun = 1;
         rr.track_reverse = 1;
-        rr.side_off = (unsigned)dyn_replay;
-        rr.tail_warps = tail_warps(replay_grid / h->sm_count);
-        rr.stage_bytes = 0;
         rr.sensor_mask = h->scene.cbs_mask;
       }
       tr<<<replay_grid, dev::kBlock, dyn_replay, stream>>>(h->d_scene, rr);

@@ -82,3 +82,17 @@ def test_the_rerun_takes_every_photon_the_cone_sees(batch, precision, cuda):
     stats, _ = run_tallies(_planes(200_003, 2, cone=True), precision, batch_photons=batch)
     assert stats["replay_launches"] == (4 if batch else 1) and stats["error_flags"] == 0
     assert stats["replayed"] == stats["detected"] == stats["hits"][0] > 100
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("make,n", [(lambda n: _planes(n, 3, cone=True), 200_003), (lambda n: _planes(n, 3), 30_001),
+                                    (lambda n: W.bilayer_rgd_mie(n, 31), 60_001), (W.mie_cbs_small, 9001)],
+                         ids=["planes_and_cone", "planes", "queue", "short_run"])
+def test_tallies_do_not_depend_on_the_route(make, n, precision, cuda):
+    """The routes' kernels round a hit's binary32 arithmetic alike: their tallies differ by
+    the order of the binary64 sums alone (1e-12 of the largest bin; another binary32 rounding
+    of every hit's products would be 1e-8 and more)."""
+    spec = make(n)
+    want = run_tallies(spec, precision)
+    for options in ({"no_replay": True}, {"blocks_per_sm": 2}, {"stage_tables": True}):
+        assert_same_run(run_tallies(spec, precision, **options), want, 1e-12)
