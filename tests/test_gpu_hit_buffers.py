@@ -85,6 +85,32 @@ def test_the_rerun_takes_every_photon_the_cone_sees(batch, precision, cuda):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_the_rerun_deposits_nothing(precision, cuda):
+    """The first walk filled the Absorption grid; the photons run again for the cone must not
+    fill it once more.  Grid: a cell's ~10^7 binary64 deposits in another order (1e-9 is 10^3
+    times their sum's random-walk error); a second deposit of the ~1 % of photons that are
+    run again is 10^6 times more."""
+    spec = _planes(200_003, 2, cone=True, absorption=True)
+    got, want = run_tallies(spec, precision), run_tallies(spec, precision, no_replay=True)
+    assert got[0]["replay_launches"] == 1 and want[0]["replay_launches"] == 0
+    assert_same_run((got[0], got[1][:-1]), (want[0], want[1][:-1]), TOL[precision])
+    np.testing.assert_allclose(got[1][-1], want[1][-1], rtol=0, atol=1e-9 * want[1][-1].max())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_a_cone_on_a_plane_above_the_surface_stays_on_the_spot(precision, cuda):
+    """Planes within 1e-9 of one another are one, at the first one's depth: a cone grouped
+    onto a plane just inside the sample can see a photon more than once, so its photons
+    cannot be listed and run again."""
+    above = {"kind": "planar_fluence", "z": 5e-10, "len_x": 4.0, "len_y": 4.0, "len_t": 0.0, "dx": 0.25,
+             "dy": 0.25, "d_t": 0.0, "absorb": False}
+    spec = _planes(200_003, 2, cone=True, first=above)
+    got, want = run_tallies(spec, precision), run_tallies(spec, precision, no_replay=True)
+    assert got[0]["replay_launches"] == 0 and got[0]["hits"][1] > 0
+    assert_same_run(got, want, 1e-12)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("make,n", [(lambda n: _planes(n, 3, cone=True), 200_003), (lambda n: _planes(n, 3), 30_001),
                                     (lambda n: W.bilayer_rgd_mie(n, 31), 60_001), (W.mie_cbs_small, 9001)],
                          ids=["planes_and_cone", "planes", "queue", "short_run"])
