@@ -964,6 +964,44 @@ static lmc_status sweep_adjoint_layout(const lmc_handle *h, const lmc_adjoint_op
 
 }  // extern "C"
 
+// Scattering events of a run's longest paths: its event cap, or where the weight in the
+// least absorbing layer meets the roulette.
+static double longest_path(const lmc_handle *h, int max_events)
+{
+  double albedo = 0.0;
+  for (int k = 0; k < h->n_scenes; ++k) {
+    const lmc::dev::Scene &sc = h->sweep ? h->scenes[k] : h->scene;
+    for (int l = 0; l < sc.n_layers; ++l)
+      albedo = std::max(albedo, sc.layers[l].albedo);
+  }
+  return albedo < 1.0 ? std::min((double)max_events, std::log(1e-4) / std::log(albedo)) : (double)max_events;
+}
+
+// Runs over planes inside the sample that are faster with every hit processed on the spot
+// than with the warps' buffers (and the CBS photons run again).  The buffers carry more
+// photons a second; but what a run cannot go below is its longest path, and an event of it
+// costs more among the 16 or 32 warps per SM of the buffered kernels than among the 8 of the
+// other (4.3 us against 2.3 in binary32), besides the rerun of the listed paths.  The more
+// photons, the more of that is hidden; the photons needed grow with the square root of the
+// longest path (their own mean path does so too).  Buffered / on the spot, ms:
+//   binary32, cone, paths to 1000: 120 k photons 8.4 / 4.8, 220 k 9.2 / 7.5, 300 k 9.8 / 11.0;
+//     to 4000: 300 k 26.4 / 22.0, 450 k 29.3 / 29.1; to 20 000: 200 k 108 / 53, 700 k 136 / 107;
+//     to 100: 80 k 0.93 / 0.78, 120 k 1.10 / 1.14
+//   binary32, no cone, to 1000: 30 k 3.3 / 3.3, 120 k 6.0 / 4.5, 220 k 6.5 / 7.1; to 20 000:
+//     30 k 40 / 45, 300 k 91 / 59, 700 k 99 / 104 (one block per SM holds 256 photons per SM:
+//     up to there both kernels run the same 8 warps)
+//   binary64, cone, to 1000: 50 k 9.2 / 7.4, 120 k 10.6 / 10.6; to 4000: 120 k 26.2 / 22.6,
+//     220 k 31.0 / 33.4; to 20 000: 300 k 123 / 114, 450 k 133 / 144; no cone: 1 k 4.1 / 5.0,
+//     50 k 5.9 / 7.2 (to 20 000 78.4 / 75.1), 1.1 M 33 / 80
+static bool spot_photons(const lmc_handle *h, bool fp32, bool cone, int max_events, uint64_t n_photons)
+{
+  const double per_sm = (double)n_photons / h->sm_count;
+  const double root = std::sqrt(longest_path(h, max_events));
+  if (cone)
+    return per_sm <= (fp32 ? 42.0 * std::max(root, 19.0) : 22.0 * root);
+  return fp32 && per_sm > 256.0 && per_sm <= 40.0 * root;
+}
+
 // Warps a block keeps to the end of a launch with per_sm blocks per SM: one for each of the
 // SM's four schedulers.
 static int tail_warps(int per_sm)
@@ -1325,13 +1363,9 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   // hits a grid reads are run again with their history.  Records keep a photon's last hit,
   // which needs its hits in order, and a CBS plane above z = 0 could list a photon twice:
   // those runs (and no_replay) process every hit on the spot.
-  // So do short runs with a CBS sensor, which the rerun would make walk their longest paths
-  // twice: buffered against on the spot, binary32 150 k photons 9.3 / 7.1 ms, 300 k 10.6 /
-  // 14.5; binary64 40 k 9.2 / 7.9, 80 k 10.3 / 10.5.  Without one the buffers are level or
-  // faster from the smallest runs on (5 k 3.4 / 3.4, 300 k 7.6 / 14.0).
-  const unsigned long long spot_photons = any_cbs ? (fp32 ? 1280ull : 512ull) * (unsigned)h->sm_count : 0;
+  // So do runs that spot_photons takes.
   const bool buffered = !h->queued && !opts->records && !opts->no_replay && !h->deep_cbs &&
-                        h->tally_doubles > 0 && n_photons > spot_photons;
+                        h->tally_doubles > 0 && !spot_photons(h, fp32, any_cbs, opts->max_events, n_photons);
   const bool rerun = buffered && any_cbs;
   rp.sensor_mask = ~0u;
   // Staged tables are a matter of the kernels with the history: with the buffers' shared
