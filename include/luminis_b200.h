@@ -238,10 +238,11 @@ typedef struct lmc_run_opts {
                                    sample                                                */
   int no_replay;                /* 1: the transport keeps every photon's reverse-path history
                                    instead of replaying the photons a FarFieldCBS grid reads
-                                   (replay is used by queued runs of more than 128 photons
-                                   per SM without records or estimator sensors, likelihood-
-                                   ratio runs included).  With planes inside the sample:
-                                   every hit processed on the spot, none buffered          */
+                                   (replay is used by queued runs without records or
+                                   estimator sensors, likelihood-ratio runs included,
+                                   except short ones whose grids read many photons, which
+                                   are faster with every history).  With planes inside the
+                                   sample: every hit processed on the spot, none buffered  */
   int tally_mode;               /* lmc_tally_mode of the hit-queue tally kernel (queued
                                    runs; inline runs add with global atomics)             */
 } lmc_run_opts;

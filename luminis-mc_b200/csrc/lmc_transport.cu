@@ -1002,6 +1002,36 @@ static bool spot_photons(const lmc_handle *h, bool fp32, bool cone, int max_even
   return fp32 && per_sm > 256.0 && per_sm <= 40.0 * root;
 }
 
+// Short runs with a FarFieldCBS sensor that are faster with every photon's history tracked
+// than with a replay of the photons a grid reads: tracked, each event of the longest path
+// costs a tenth (binary32) to a fifth more; the replay walks the longest path it finds among
+// its M photons once again, at that cost.  Paths longer than k events are as rare as
+// 1 / sqrt(k), so that path is long enough from an M ~ sqrt(longest path) on.  M from the solid
+// angle of the grid, as if a diffuse surface sent every photon back.  Tracked / replayed, ms:
+//   paths to 1000, cone of 0.1 rad: 300 photons binary64 3.95 / 3.26, binary32 2.66 / 2.39;
+//     1 k 3.47 / 3.70, 2.14 / 2.68; 10 k 3.53 / 4.84, 2.19 / 3.29
+//   to 9200, 0.1 rad: 300 photons 27.2 / 24.9, 17.0 / 16.7; 1 k 30.4 / 35.8, 19.2 / 19.2
+//   to 20 000, 0.02 rad: 18 k photons 63.5 / 56.4, 39.3 / 36.2; 0.1 rad: 1 k 60.6 / 59.2,
+//     38.6 / 36.3; 3 k 62.6 / 80.7, 38.7 / 38.4; 0.5 rad: 300 photons 60.6 / 79.9, 37.5 / 47.4
+//   derivatives, sweep of 32 media: 300 photons 4.5 / 3.2, 18 k 4.2 / 4.5
+// With more photons than a short run's the replay costs its fixed 1.1 ms, tracking a growing
+// share (1 M photons: 13.1 against 15.3 ms); between the two the default stays with the replay.
+static bool tracked_photons(const lmc_handle *h, int max_events, uint64_t n_photons)
+{
+  double share = 0.0;
+  for (int k = 0; k < h->n_scenes; ++k) {
+    const lmc::dev::Scene &sc = h->sweep ? h->scenes[k] : h->scene;
+    for (int i = 0; i < sc.n_sensors; ++i) {
+      const lmc::dev::Sensor &s = sc.sensors[i];
+      if (!((sc.cbs_mask >> i) & 1u))
+        continue;
+      const double sin_max = std::sin(std::min(s.N_theta * s.dtheta, 0.5 * M_PI));
+      share = std::max(share, sin_max * sin_max * std::min(1.0, s.N_phi * s.dphi / (2.0 * M_PI)));
+    }
+  }
+  return (double)n_photons * share >= 0.1 * std::sqrt(longest_path(h, max_events));
+}
+
 // Warps a block keeps to the end of a launch with per_sm blocks per SM: one for each of the
 // SM's four schedulers.
 static int tail_warps(int per_sm)
@@ -1327,11 +1357,8 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
       dyn_tally = (size_t)(1 + rp.adj_K) * (adj->radial_bins + 1) * sizeof(double);
   }
   // At most one warp per scheduler: the run lasts as long as its longest path, and every
-  // instruction of an event counts as latency.  The 2-block variant (no spills) with the
-  // history tracked then beats the 4-block one and a replay that walks the longest hits'
-  // paths once more: 10 k CBS photons 3.4 -> 2.2 ms (binary64 5.5 -> 3.5).  With more photons
-  // the replay costs its fixed 1.1 ms, tracking a growing share (1 M photons: 13.1 against
-  // 15.3 ms); between the two the default stays with the replay.
+  // instruction of an event counts as latency: the 2-block variant (no spills) beats the
+  // 4-block one (20 000 events: 35.1 ms against 36.9).
   const bool short_run = n_photons <= 128ull * (unsigned)h->sm_count;
   // binary32 queued transport: a 4-block (<=64 registers, the default) and a
   // 2-block (<=128 registers) variant; blocks_per_sm == 1 or 2 selects the latter
@@ -1356,8 +1383,8 @@ static lmc_status run_impl(lmc_handle *h, uint64_t seed, uint64_t photon_begin, 
   bool any_cbs = false;
   for (int k = 0; k < h->n_scenes; ++k)
     any_cbs = any_cbs || (sw ? h->scenes[k] : h->scene).cbs_mask != 0;
-  const bool replay = h->queued && !est && !opts->records && !opts->no_replay && !short_run &&
-                      opts->track_reverse_paths && any_cbs;
+  const bool replay = h->queued && !est && !opts->records && !opts->no_replay && opts->track_reverse_paths &&
+                      any_cbs && !(short_run && tracked_photons(h, opts->max_events, n_photons));
   rp.cbs_replay = replay ? 1 : 0;
   // Planes inside the sample: hits go through the warps' buffers, and the photons whose CBS
   // hits a grid reads are run again with their history.  Records keep a photon's last hit,
