@@ -186,7 +186,7 @@ constexpr int kAdjMaxRadialBins = 512;
 struct Queue {
   unsigned long long cap;
   void *entry;                           // HitEntry<R>[cap]
-  void *r;                               // R[kQRFields + scores][cap]; null: no hit has them
+  void *r;                               // R[kQRFields + scores][cap] (warps' buffers: none)
 };
 
 // kHitsBuffer: a photon whose exit a FarFieldCBS grid sees, listed to be run again, with
